@@ -147,6 +147,14 @@ SIGNATURES = {
     "ghexb_plan_rebind": [_vp, C.POINTER(_vp), _i, _vp],
     "ghexb_stencil7": [_i, _i, C.POINTER(_vp), C.POINTER(_vp), C.POINTER(C.c_int64), C.POINTER(C.c_int64), _i,
                        C.c_double, _i, _vp],
+    "ghexb_program_create": [C.POINTER(_vp), _i, _i, C.POINTER(_vp)],
+    "ghexb_program_destroy": [_vp],
+    "ghexb_program_buffer_bytes": [_vp, _pi64],
+    "ghexb_program_steps": [_vp, C.POINTER(_vp), _vp, C.POINTER(_vp), _vp, _vp, _i, C.c_double, _i, _i, _vp],
+    "ghexb_sumsq_partials": [_i, _i, _pi64, _i, _pi64],
+    "ghexb_sumsq": [_i, _i, C.POINTER(_vp), C.POINTER(C.c_int64), C.POINTER(C.c_int64), _i, _vp, _i64, _vp, _vp],
+    "ghexb_program_sumsq": [_vp, _vp, _vp, _i64, _vp, _vp],
+    "ghexb_sumsq_grad": [_i, _i, C.POINTER(_vp), C.POINTER(_vp), C.POINTER(C.c_int64), C.POINTER(C.c_int64), _i, _vp, _vp],
 }
 
 for _name, _args in SIGNATURES.items():

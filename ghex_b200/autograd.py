@@ -24,6 +24,7 @@ rewrite of the descriptor tables). Plans hold no references to the tensors they 
 from __future__ import annotations
 
 import ctypes as C
+import math
 from collections import OrderedDict
 from typing import Any, Sequence
 
@@ -83,6 +84,7 @@ class DifferentiableExchange:
         self.graph = graph
         self._fwd = _PlanPool(ctx, self._bis, pool)
         self._bwd = _PlanPool(ctx, self._bis, pool)
+        self._programs: dict = {}
 
     def __len__(self) -> int:
         return len(self._layout)
@@ -114,6 +116,22 @@ class DifferentiableExchange:
         self.check(grads)
         stream = torch.cuda.current_stream(grads[0].device)
         self._bwd.get(grads, stream).adjoint(stream=stream)
+
+    def _program(self, halo: int):
+        """The exchange and the 7-point update in fused passes, or None for an exchange that
+        ghexb_program_create refuses (then the two run one after the other)."""
+        if halo not in self._programs:
+            program = None
+            dense = all(torch.empty_like(t).stride() == t.stride() for t in
+                        (torch.empty_strided(sh, st, dtype=dt, device="meta") for sh, st, dt, _ in self._tensor_layout))
+            if dense and len({dev for *_, dev in self._tensor_layout}) == 1 and self._tensor_layout[0][3].type == "cuda":
+                try:
+                    program = _Program(self._bis, halo)
+                except _capi.GhexError as e:
+                    if e.code != _capi.ERR_INVALID:
+                        raise
+            self._programs[halo] = program
+        return self._programs[halo]
 
     def __call__(self, *tensors: torch.Tensor):
         if len(tensors) == 1 and isinstance(tensors[0], (list, tuple)):
@@ -201,34 +219,172 @@ def stencil7(xs: Sequence[torch.Tensor], alpha: float = 0.1, halo: int = 1):
     return out if isinstance(out, tuple) else (out,)
 
 
+class _Program:
+    """The fused passes of one exchange (ghexb_program_*)."""
+
+    def __init__(self, bis: Sequence[BufferInfo], halo: int):
+        handles = (C.c_void_p * len(bis))(*[bi.handle() for bi in bis])
+        h = C.c_void_p()
+        call("ghexb_program_create", handles, len(bis), halo, C.byref(h))
+        self._h = h
+        n = C.c_int64()
+        call("ghexb_program_buffer_bytes", h, C.byref(n))
+        self.buffer_bytes = n.value
+
+    def buffer(self, device) -> torch.Tensor:
+        return torch.empty(self.buffer_bytes, dtype=torch.uint8, device=device)
+
+    def steps(self, steps: int, alpha: float, stream, *, fields=None, source=None, out=None, a=None, b=None,
+              adjoint: bool = False, twice: bool = False) -> None:
+        def array(tensors):
+            return None if tensors is None else (C.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+        def address(t):
+            return None if t is None else t.data_ptr()
+        call("ghexb_program_steps", self._h, array(fields), address(source), array(out), address(a), address(b), steps,
+             float(alpha), int(adjoint), int(twice), C.c_void_p(stream.cuda_stream))
+
+    def __del__(self, _release=_capi.release):
+        _release("ghexb_program_destroy", getattr(self, "_h", None))
+        self._h = None
+
+
+class _Diffusion(torch.autograd.Function):
+    """The program as one function: the exchange of the given tensors (their halos are the
+    caller's to see), then one fused pass a step."""
+
+    @staticmethod
+    def forward(ctx, dx: DifferentiableExchange, program: _Program, steps: int, alpha: float, halo: int, *xs):
+        dx.exchange_(xs)
+        dev = xs[0].device
+        outs = [torch.empty_like(x) for x in xs]
+        a, b = (program.buffer(dev) if steps > k else None for k in (1, 2))
+        program.steps(steps, alpha, torch.cuda.current_stream(dev), fields=xs, out=outs, a=a, b=b)
+        ctx.dx, ctx.program, ctx.steps, ctx.alpha, ctx.halo = dx, program, steps, alpha, halo
+        ctx.mark_dirty(*xs)
+        ctx.set_materialize_grads(False)
+        return (*xs, *outs)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        dx, program, steps, alpha = ctx.dx, ctx.program, ctx.steps, ctx.alpha
+        n = len(dx)
+        exchanged, gys = grads[:n], grads[n:]
+        layouts = dx._tensor_layout
+        dev = layouts[0][3]
+
+        def like_fields(g, shape, stride, dtype, device):
+            if g is not None and g.shape == shape and g.stride() == stride and g.dtype == dtype:
+                return g
+            buf = torch.empty_strided(shape, stride, dtype=dtype, device=device)
+            return buf.zero_() if g is None else buf.copy_(g)
+
+        def new():
+            return [torch.empty_strided(shape, stride, dtype=dtype, device=device) for shape, stride, dtype, device in layouts]
+        g = [like_fields(g, *lay) for g, lay in zip(gys, layouts)]
+        stream = torch.cuda.current_stream(dev)
+        seen = any(e is not None for e in exchanged)  # the exchanged inputs were used as well: the first step in two parts
+        fused = steps - 1 if seen else steps
+        if fused:
+            outs = new()
+            a, b = (program.buffer(dev) if fused > k else None for k in (1, 2))
+            program.steps(fused, alpha, stream, fields=g, out=outs, a=a, b=b, adjoint=True)
+            g = outs
+        if seen:
+            outs = new()
+            _launch_stencil(g, outs, alpha, ctx.halo, adjoint=True)
+            for o, e in zip(outs, exchanged):
+                if e is not None:
+                    o += e
+            dx.adjoint_(outs)
+            g = outs
+        return (None, None, None, None, None, *g)
+
+
 def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], steps: int = 10, alpha: float = 0.1,
                       halo: int = 1):
     """steps x (halo exchange, 7-point update); returns the final fields. The first exchange
-    writes into xs: pass clones of leaf tensors that require grad."""
+    writes into xs: pass clones of leaf tensors that require grad. Where the exchange allows it,
+    a step is one kernel (same bits)."""
     xs = tuple(xs)
+    if steps > 0 and type(dx) is DifferentiableExchange and math.isfinite(alpha):
+        program = dx._program(halo)
+        if program is not None:
+            return _Diffusion.apply(dx, program, steps, alpha, halo, *xs)[len(xs):]
     for _ in range(steps):
         xs = dx(*xs)
         xs = stencil7(xs, alpha, halo)
     return xs
 
 
+def _plain(xs) -> bool:
+    """Ordinary CUDA tensors outside every transform and mode that sees torch's own operations
+    (functorch, forward-mode AD, dispatch modes, tracing)."""
+    return (all(type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.layout == torch.strided and not x.is_neg()
+                and not torch._C._functorch.is_functorch_wrapped_tensor(x) for x in xs)
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._len_torch_dispatch_stack() == 0
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing())
+
+
+def _array_args(xs) -> tuple:
+    n = len(xs)
+    return (_capi.F64 if xs[0].dtype == torch.float64 else _capi.F32, n, (C.c_void_p * n)(*[x.data_ptr() for x in xs]),
+            (C.c_int64 * (3 * n))(*[e for x in xs for e in x.shape]), (C.c_int64 * (3 * n))(*[s for x in xs for s in x.stride()]))
+
+
+class _SumSquares(torch.autograd.Function):
+    """The sum of squares of the interiors, and its gradient, as kernels over all domains."""
+
+    @staticmethod
+    def forward(ctx, halo: int, *xs):
+        dtype, n, ptrs, ext, st = _array_args(xs)
+        count = C.c_int64()
+        call("ghexb_sumsq_partials", dtype, n, ext, halo, C.byref(count))
+        partials = torch.empty(count.value, dtype=torch.float64, device=xs[0].device)
+        out = torch.empty((), dtype=xs[0].dtype, device=xs[0].device)
+        stream = torch.cuda.current_stream(xs[0].device).cuda_stream
+        call("ghexb_sumsq", dtype, n, ptrs, ext, st, halo, C.c_void_p(partials.data_ptr()), count.value,
+             C.c_void_p(out.data_ptr()), C.c_void_p(stream))
+        ctx.save_for_backward(*xs)
+        ctx.halo = halo
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        xs, h = ctx.saved_tensors, ctx.halo
+        if torch.is_grad_enabled():  # a gradient that is differentiated in turn: in torch's operations
+            return (None, *[torch.nn.functional.pad(g * (2 * x[h:-h, h:-h, h:-h]), (h,) * 6) for x in xs])
+        dtype, n, ptrs, ext, st = _array_args(xs)
+        outs = [torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) for x in xs]
+        stream = torch.cuda.current_stream(xs[0].device).cuda_stream
+        call("ghexb_sumsq_grad", dtype, n, ptrs, (C.c_void_p * n)(*[o.data_ptr() for o in outs]), ext, st, h,
+             C.c_void_p(g.data_ptr()), C.c_void_p(stream))
+        return (None, *outs)
+
+
 def interior_loss(xs: Sequence[torch.Tensor], halo: int = 1) -> torch.Tensor:
     """Sum of squares of the interiors."""
     h = halo
+    xs = tuple(xs)
+    if xs and h >= 1 and _plain(xs) and all(
+            x.dim() == 3 and x.dtype in (torch.float32, torch.float64) and x.dtype == xs[0].dtype and x.device == xs[0].device
+            and min(x.shape) > 2 * h and min(x.stride()) > 0 for x in xs):
+        return _SumSquares.apply(h, *xs)
     return sum((x[h:-h, h:-h, h:-h] ** 2).sum() for x in xs)
 
 
 class GraphedDiffusion:
     """The diffusion program (``steps`` x (halo exchange, 7-point update), loss = sum of squares of
     the final interiors) and its gradient with respect to the input fields, replayed from one CUDA
-    graph: the kernels of ``diffusion_program`` and of its backward through torch.autograd, in the
-    same order, on buffers of fixed memory, so that the host launches one graph instead of the
-    program's kernels one by one.
+    graph on buffers of fixed memory, with the bits of ``diffusion_program``, ``interior_loss`` and
+    their backward through torch.autograd.
 
-    The forward alternates two buffer sets; the backward seeds 2 x (final interior) and applies, for
-    every step in reverse, the stencil's transpose and then the exchange's adjoint, on two more
-    buffer sets. Four exchange plans of its own are bound to the four sets before the capture, so
-    the capture holds only kernel launches. ``run(xs)`` copies the inputs in, replays the graph, and returns the loss and
+    Where the exchange allows fused passes, a step is one kernel, forward and backward: the first
+    one reads the inputs where they are (a launch of its own before the replay), the others are the
+    graph's. Otherwise the graph holds the exchange and update kernels: the forward alternates two
+    buffer sets; the backward seeds 2 x (final interior) and applies, for every step in reverse, the
+    stencil's transpose and then the exchange's adjoint, on two more buffer sets, with four exchange
+    plans of its own bound to the four sets before the capture. ``run(xs)`` returns the loss and
     the gradient (tensors the next run overwrites)."""
 
     def __init__(self, dx: DifferentiableExchange, templates: Sequence[torch.Tensor], steps: int = 10,
@@ -237,6 +393,10 @@ class GraphedDiffusion:
         dx.check(templates)
         self.dx, self.steps, self.alpha, self.halo = dx, steps, alpha, halo
         dev = templates[0].device
+        self._program = dx._program(halo) if steps > 0 and math.isfinite(alpha) else None
+        if self._program is not None:
+            self._capture_fused(templates, dev)
+            return
 
         def buffers():
             return [torch.zeros_like(t) for t in templates]
@@ -260,6 +420,32 @@ class GraphedDiffusion:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, stream=stream):
             self.loss, self.grad = self._body()
+
+    def _capture_fused(self, templates, dev) -> None:
+        if ExchangePlan(self.dx.context, self.dx._bis).info()["adjoint_launches"] != 1:
+            raise ValueError("a graphed program needs an exchange whose adjoint is one kernel")
+        program, steps, alpha = self._program, self.steps, self.alpha
+        self._layout = [(t.shape, t.stride(), t.dtype, t.device) for t in templates]
+        self._inp = None
+        self._packed = [program.buffer(dev) for _ in range(2)]
+        self.grad = [torch.zeros_like(t) for t in templates]
+        self.loss = torch.zeros((), dtype=templates[0].dtype, device=dev)
+        dtype, n, _, ext, _ = _array_args(templates)
+        count = C.c_int64()
+        call("ghexb_sumsq_partials", dtype, n, ext, self.halo, C.byref(count))
+        self._partials = torch.empty(count.value, dtype=torch.float64, device=dev)
+        a, b = self._packed
+        final = a if steps % 2 else b
+        stream = torch.cuda.Stream(device=dev)
+        stream.wait_stream(torch.cuda.current_stream(dev))
+        torch.cuda.synchronize(dev)
+        self.graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(self.graph, stream=stream):  # the first step has written a
+            if steps > 1:
+                program.steps(steps - 1, alpha, stream, source=a, a=a, b=b)
+            call("ghexb_program_sumsq", program._h, final.data_ptr(), self._partials.data_ptr(), count.value,
+                 self.loss.data_ptr(), C.c_void_p(stream.cuda_stream))
+            program.steps(steps, alpha, stream, source=final, out=self.grad, a=a, b=b, adjoint=True, twice=True)
 
     def _body(self):
         s = torch.cuda.current_stream()
@@ -288,7 +474,19 @@ class GraphedDiffusion:
         return loss, g
 
     def run(self, xs: Sequence[torch.Tensor]):
-        for y, x in zip(self._inp, xs):
-            y.copy_(x)
+        if self._program is not None:
+            xs = list(xs)
+            if len(xs) != len(self._layout) or not all(
+                    type(x) in (torch.Tensor, torch.nn.Parameter) and (x.shape, x.stride(), x.dtype, x.device) == lay
+                    and not x.is_neg() for x, lay in zip(xs, self._layout)):
+                if self._inp is None:  # inputs of another layout are copied into the fields' layout first
+                    self._inp = [torch.zeros_like(g) for g in self.grad]
+                for y, x in zip(self._inp, xs):
+                    y.copy_(x)
+                xs = self._inp
+            self._program.steps(1, self.alpha, torch.cuda.current_stream(xs[0].device), fields=xs, a=self._packed[0])
+        else:
+            for y, x in zip(self._inp, xs):
+                y.copy_(x)
         self.graph.replay()
         return self.loss, self.grad

@@ -3,6 +3,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -14,6 +15,7 @@
 #include "ipc.hpp"
 #include "kernels.hpp"
 #include "plan.hpp"
+#include "program.hpp"
 #include "stencil.hpp"
 
 namespace
@@ -1045,6 +1047,151 @@ int ghexb_stencil7(int dtype, int n, const void* const* in, void* const* out, co
         ghexb::check_cuda(ghexb::launch_stencil7(dtype == GHEXB_F64, doms.data(), n, alpha, adjoint != 0,
                               static_cast<cudaStream_t>(stream)),
             "stencil launch");
+    });
+}
+
+// ---- the program in fused passes -------------------------------------------------------------
+int ghexb_program_create(const ghexb_field* fields, int n, int halo, ghexb_program* out)
+{
+    return guarded([&] {
+        require(fields && out, "null argument");
+        require(n > 0, "a program needs at least one field");
+        for (int i = 0; i < n; ++i) require(fields[i] != nullptr, "null field handle");
+        auto p = std::make_unique<ghexb_program_s>();
+        ghexb::build_program(*p, fields, n, halo);
+        *out = p.release();
+    });
+}
+
+int ghexb_program_destroy(ghexb_program program)
+{
+    delete program;
+    return GHEXB_OK;
+}
+
+int ghexb_program_buffer_bytes(ghexb_program program, int64_t* bytes)
+{
+    return guarded([&] {
+        require(program && bytes, "null argument");
+        *bytes = program->packed_elements * (program->f64 ? 8 : 4);
+    });
+}
+
+int ghexb_program_steps(ghexb_program program, const void* const* fields, const void* source, void* const* out, void* a,
+    void* b, int steps, double alpha, int adjoint, int twice, void* stream)
+{
+    return guarded([&] {
+        require(program != nullptr, "null argument");
+        require(steps >= 1, "a program runs at least one step");
+        require((fields != nullptr) != (source != nullptr), "either the fields or a packed source is needed");
+        require(!twice || (adjoint && source), "only a packed source of the transpose is doubled");
+        const size_t n = program->domains.size(), es = program->f64 ? 8 : 4;
+        const auto aligned = [](const void* p, size_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; };
+        for (size_t i = 0; i < n; ++i)
+        {
+            require(!fields || (fields[i] && aligned(fields[i], es)), "a field is null or not aligned to its element size");
+            require(!out || (out[i] && aligned(out[i], es)), "an output is null or not aligned to its element size");
+            // the output of a single pass must not be its input
+            require(!fields || !out || steps > 1 || fields[i] != out[i], "input and output overlap");
+        }
+        const int packed = steps - (out ? 1 : 0); // passes that write a packed buffer
+        require(packed < 1 || ((source == a ? b : a) != nullptr), "a packed buffer is missing");
+        require(packed < 2 || (a && b && a != b), "two packed buffers are needed");
+        require(aligned(a, 16) && aligned(b, 16) && aligned(source, 16), "packed buffers are 16-byte aligned");
+        ghexb::check_cuda(ghexb::launch_passes(*program, fields, source, out, a, b, steps, alpha, adjoint != 0, twice != 0,
+                              static_cast<cudaStream_t>(stream)),
+            "program launch");
+    });
+}
+
+namespace
+{
+// the interiors (or, whole, the arrays) of n 3-D arrays, checked as ghexb_stencil7's
+std::vector<ghexb::interior> interiors(int dtype, int n, const void* const* in, const int64_t* extents, const int64_t* strides,
+    int halo, bool whole)
+{
+    require(in && extents && strides, "null argument");
+    require(dtype == GHEXB_F32 || dtype == GHEXB_F64, "the sum of squares needs float32 or float64");
+    require(n >= 0 && halo >= 1, "negative domain count, or a halo of width < 1");
+    const int64_t es = dtype == GHEXB_F64 ? 8 : 4;
+    std::vector<ghexb::interior> d(n);
+    for (int i = 0; i < n; ++i)
+    {
+        require(in[i] && reinterpret_cast<uintptr_t>(in[i]) % es == 0, "a data pointer is null or not aligned to its element size");
+        int64_t off = 0, cells = 1;
+        for (int a = 0; a < 3; ++a)
+        {
+            const int64_t e = extents[3 * i + a], s = strides[3 * i + a];
+            require(e > 2 * halo && e < (int64_t(1) << 30), "every extent must exceed twice the halo width");
+            require(s > 0, "strides must be positive");
+            cells *= e;
+            require(cells < (int64_t(1) << 42), "an array of 2^42 elements");
+            d[i].n[a] = (int32_t)(whole ? e : e - 2 * halo), d[i].s[a] = s;
+            off += whole ? 0 : halo * s;
+        }
+        require((int64_t)d[i].n[1] * d[i].n[2] < (int64_t(1) << 31), "an array of 2^31 rows");
+        d[i].p = static_cast<const char*>(in[i]) + off * es;
+    }
+    return d;
+}
+
+int64_t partials_of(bool f64, const std::vector<ghexb::interior>& d)
+{
+    std::vector<std::array<int32_t, 3>> e;
+    for (const auto& s : d) e.push_back({s.n[0], s.n[1], s.n[2]});
+    return e.empty() ? 0 : ghexb::sumsq_blocks(f64, reinterpret_cast<const int32_t(*)[3]>(e.data()), (int)e.size());
+}
+} // namespace
+
+int ghexb_sumsq_partials(int dtype, int n, const int64_t* extents, int halo, int64_t* count)
+{
+    return guarded([&] {
+        require(count != nullptr, "null argument");
+        const std::vector<const void*> at(n > 0 ? n : 0, reinterpret_cast<const void*>(uintptr_t(64)));
+        const std::vector<int64_t> ones(3 * (size_t)(n > 0 ? n : 0), 1);
+        const void* none = nullptr;
+        const int64_t one = 1;
+        *count = partials_of(dtype == GHEXB_F64,
+            interiors(dtype, n, n > 0 ? at.data() : &none, extents, n > 0 ? ones.data() : &one, halo, false));
+    });
+}
+
+int ghexb_sumsq(int dtype, int n, const void* const* in, const int64_t* extents, const int64_t* strides, int halo,
+    double* partials, int64_t count, void* out, void* stream)
+{
+    return guarded([&] {
+        const auto d = interiors(dtype, n, in, extents, strides, halo, false);
+        require(n > 0 && partials && out, "null argument");
+        require(count >= partials_of(dtype == GHEXB_F64, d), "too little room for the partial sums");
+        ghexb::check_cuda(ghexb::launch_sumsq(dtype == GHEXB_F64, d.data(), n, false, partials, out, static_cast<cudaStream_t>(stream)),
+            "sum of squares launch");
+    });
+}
+
+int ghexb_program_sumsq(ghexb_program program, const void* source, double* partials, int64_t count, void* out, void* stream)
+{
+    return guarded([&] {
+        require(program && source && partials && out, "null argument");
+        require(reinterpret_cast<uintptr_t>(source) % 16 == 0, "packed buffers are 16-byte aligned");
+        std::vector<ghexb::interior> d;
+        for (const auto& p : program->domains)
+            d.push_back({static_cast<const char*>(source) + p.offset * (program->f64 ? 8 : 4), {p.n[0], p.n[1], p.n[2]}, {1, p.row, p.plane}});
+        require(count >= partials_of(program->f64, d), "too little room for the partial sums");
+        ghexb::check_cuda(ghexb::launch_sumsq(program->f64, d.data(), (int)d.size(), true, partials, out, static_cast<cudaStream_t>(stream)),
+            "sum of squares launch");
+    });
+}
+
+int ghexb_sumsq_grad(int dtype, int n, const void* const* in, void* const* out, const int64_t* extents, const int64_t* strides,
+    int halo, const void* g, void* stream)
+{
+    return guarded([&] {
+        const auto d = interiors(dtype, n, in, extents, strides, halo, true);
+        require(out && g, "null argument");
+        for (int i = 0; i < n; ++i) require(out[i] && out[i] != in[i], "an output is null or its input");
+        if (n == 0) return;
+        ghexb::check_cuda(ghexb::launch_sumsq_grad(dtype == GHEXB_F64, d.data(), out, n, halo, g, static_cast<cudaStream_t>(stream)),
+            "sum of squares launch");
     });
 }
 

@@ -1,0 +1,835 @@
+// The differentiable program (halo exchange, 7-point update, repeated; and its transpose) in one
+// kernel per step.
+//
+// Between the first and the last step nobody sees the halos, so a pass does not fill them: a cell
+// next to a domain's face takes the neighbour's interior cell that the exchange would have copied
+// beside it, and the transpose adds, after the cell's own value, the contribution that the
+// exchange's adjoint would have added from each of its images, in the same order. Every value is
+// the one that the exchange kernel and the stencil kernel (stencil.cu) compute one after the
+// other, with the same roundings, so results have the same bits.
+//
+// The fields between two passes are the program's own, and packed: interiors only, rows on
+// 32-byte boundaries, so that a thread moves 16 bytes at a time whatever the domains' extents.
+//
+// One step on 8 domains of 128 x 128 x 64, as exchange + update kernels and as a pass: forward
+// 6.6 + 42.3 us and 27.9 us in float64, 5.5 + 31.2 us and 13.7 us in float32; transposed 8.6 +
+// 42.9 us and 43.3 us, 7.9 + 28.1 us and 23.4 us. The floor, one read and one write of every cell
+// at the HBM rate, is 20.5 and 10.2 us.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <map>
+#include <string>
+#include <utility>
+
+#include "program.hpp"
+
+namespace ghexb
+{
+namespace
+{
+template <typename T> __device__ __forceinline__ T add_rn(T a, T b);
+template <typename T> __device__ __forceinline__ T sub_rn(T a, T b);
+template <typename T> __device__ __forceinline__ T mul_rn(T a, T b);
+template <> __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+template <> __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+template <> __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+template <> __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+template <> __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+template <> __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+
+// x + alpha * (s - 6 x), s the sum of the six neighbours (stencil.cu)
+template <typename T> __device__ __forceinline__ T update(T x, T s, T alpha)
+{
+    return add_rn(x, mul_rn(alpha, sub_rn(s, mul_rn(T(6), x))));
+}
+
+// 16 bytes of consecutive cells
+template <typename T> struct alignas(16) cells
+{
+    static constexpr int V = 16 / (int)sizeof(T);
+    T v[V];
+};
+
+constexpr int k_batch = 32; // domains per launch
+
+// One domain of a launch; cell (0, 0, 0) is the first interior cell, strides count elements.
+struct pass_domain
+{
+    const void* in;
+    void* out;
+    int32_t nx, ny, nz, halo;
+    int32_t isx, isy, isz, osx, osy, osz;
+    struct
+    {
+        const void* p; // the cells beyond the face: p[u * s0 + v * s1], (u, v) the other axes in order
+        int32_t s0, s1;
+    } f[6];
+    uint32_t ranks, images;
+    uint32_t chunks, slab, columns, groups; // chunks a row, planes a slab, columns (chunks x strips), blocks a slab
+    uint32_t block0, marches; // first block; blocks that march (the others write the halo)
+};
+struct pass_args
+{
+    pass_domain d[k_batch];
+    int n;
+};
+
+// A thread marches along z through a slab of planes of a column of 16 bytes of consecutive cells
+// (x) by `rows` rows (y); consecutive threads take consecutive cells of a row, then the next strip
+// of rows, so no thread idles but in a row's last chunk. The planes it reads (its rows, the row
+// before and after them and the cells beside them) pass through a ring of its own in shared
+// memory, filled by asynchronous copies k_stages - 1 planes ahead; nothing is shared between
+// threads, so there is no barrier, and the rows and cells that neighbouring threads read too come
+// from L1 or L2.
+constexpr int k_threads = 128;
+constexpr int k_rows = 2;
+constexpr int k_stages = 3;
+constexpr int k_resident = 5; // blocks per SM
+constexpr int k_min_slab = 4; // planes
+constexpr int k_halo_cells = 8; // halo cells a thread writes
+
+// a plane in the ring of a block: rows -1 .. R of 16 bytes per thread, then the cells beside the R rows
+template <typename T> struct ring
+{
+    static constexpr int wide = 16 * k_threads, narrow = (int)sizeof(T) * k_threads;
+    static constexpr int stage = (k_rows + 2) * wide + 2 * k_rows * narrow;
+    static constexpr int bytes = k_stages * stage;
+};
+
+template <int N> __device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool valid)
+{
+    // src-size 0 writes zeros and reads nothing
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(N), "r"(valid ? N : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <typename T, bool ADJOINT, bool TWICE>
+__device__ __forceinline__ void write_halo(const pass_domain& d, T alpha, uint32_t block)
+{
+    const int h = d.halo, nx = d.nx, ny = d.ny, nz = d.nz;
+    const uint32_t ex = nx + 2 * h, ey = ny + 2 * h;
+    const uint32_t zcells = ex * ey * (2 * h), ycells = ex * (2 * h) * nz, xcells = (2 * h) * ny * nz;
+    const T* __restrict__ in = static_cast<const T*>(d.in);
+    T* __restrict__ out = static_cast<T*>(d.out);
+    for (int q = 0; q < k_halo_cells; ++q)
+    {
+        uint32_t c = (block * k_halo_cells + q) * k_threads + threadIdx.x;
+        int i, j, k;
+        if (c < zcells)
+        {
+            const uint32_t r = c / ex, v = r / ey;
+            i = (int)(c - r * ex) - h, j = (int)(r - v * ey) - h;
+            k = (int)v < h ? (int)v - h : nz + (int)v - h;
+        }
+        else if ((c -= zcells) < ycells)
+        {
+            const uint32_t r = c / ex, v = r / (2 * h);
+            i = (int)(c - r * ex) - h, k = (int)v;
+            j = (int)(r - v * (2 * h));
+            j = j < h ? j - h : ny + j - h;
+        }
+        else if ((c -= ycells) < xcells)
+        {
+            const uint32_t r = c / (2 * h), v = r / ny;
+            i = (int)(c - r * (2 * h)), j = (int)(r - v * ny), k = (int)v;
+            i = i < h ? i - h : nx + i - h;
+        }
+        else
+            return;
+        T y = T(0);
+        if constexpr (ADJOINT)
+        {
+            const int region = (i < 0 ? 0 : i < nx ? 1 : 2) + 3 * (j < 0 ? 0 : j < ny ? 1 : 2) + 9 * (k < 0 ? 0 : k < nz ? 1 : 2);
+            if (!((d.images >> region) & 1u)) // a halo cell that nothing was copied to keeps its gradient
+            {
+                const auto G = [&](int a, int b, int e) {
+                    if (a < 0 || a >= nx || b < 0 || b >= ny || e < 0 || e >= nz) return T(0);
+                    const T g = __ldg(in + (a * d.isx + b * d.isy + e * d.isz));
+                    return TWICE ? mul_rn(T(2), g) : g;
+                };
+                T t = add_rn(G(i - 1, j, k), G(i + 1, j, k));
+                t = add_rn(t, G(i, j - 1, k));
+                t = add_rn(t, G(i, j + 1, k));
+                t = add_rn(t, G(i, j, k - 1));
+                t = add_rn(t, G(i, j, k + 1));
+                y = update(T(0), t, alpha);
+            }
+        }
+        out[i * d.osx + j * d.osy + k * d.osz] = y;
+    }
+}
+
+template <typename T, bool ADJOINT, bool TWICE, bool IN_PACKED, bool OUT_PACKED>
+__global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __grid_constant__ pass_args args, T alpha)
+{
+    constexpr int V = cells<T>::V, R = k_rows;
+    uint32_t b = blockIdx.x;
+    int di = 0;
+    while (di + 1 < args.n && b >= args.d[di + 1].block0) ++di;
+    const pass_domain& d = args.d[di];
+    b -= d.block0;
+    if (b >= d.marches)
+    {
+        if constexpr (!OUT_PACKED) write_halo<T, ADJOINT, TWICE>(d, alpha, b - d.marches);
+        return;
+    }
+    const int nx = d.nx, ny = d.ny, nz = d.nz;
+    const uint32_t bz = b / d.groups, t = (b - bz * d.groups) * k_threads + threadIdx.x;
+    const bool live = t < d.columns; // the others only take part in the shuffles
+    const uint32_t column = live ? t : d.columns - 1, strip = column / d.chunks;
+    const int k0 = (int)(bz * d.slab), k1 = min(nz, k0 + (int)d.slab);
+    const int i0 = (int)(column - strip * d.chunks) * V, m = min(V, nx - i0);
+    const int j0 = min((int)strip * R, ny - R); // the last strip overlaps the one before (same values)
+    const T* __restrict__ in = static_cast<const T*>(d.in);
+    T* __restrict__ out = static_cast<T*>(d.out);
+    const int sx = IN_PACKED ? 1 : d.isx, sy = d.isy, sz = d.isz;
+    const bool first = i0 == 0, last = i0 + V >= nx; // the chunk touches face x-, x+
+    const int lane = threadIdx.x & 31;
+
+    const T* const c0 = in + (i0 * sx + j0 * sy);
+    // the rows before and after the strip and the cells beside it, in the column's own domain or
+    // beyond a face (nullptr: zeros)
+    const T *lo = c0 - sy, *hi = c0 + R * sy;
+    int lo_x = sx, lo_z = sz, hi_x = sx, hi_z = sz;
+    const auto face = [&](int f) { return static_cast<const T*>(d.f[f].p); };
+    const bool front = j0 == 0, back = j0 + R == ny; // the strip touches face y-, y+
+    if (front) lo = face(2) ? face(2) + i0 * d.f[2].s0 : nullptr, lo_x = d.f[2].s0, lo_z = d.f[2].s1;
+    if (back) hi = face(3) ? face(3) + i0 * d.f[3].s0 : nullptr, hi_x = d.f[3].s0, hi_z = d.f[3].s1;
+    // a neighbouring lane holds the cell beside a row but at the ends of the row and of the warp,
+    // where a thread reads the cell itself: the left one, or the right one, seldom both
+    struct side_cells
+    {
+        const T* p;
+        int y, z;
+    };
+    const bool need_left = first || lane == 0, need_right = last || lane == 31, need_both = need_left && need_right;
+    const auto left_cells = [&]() -> side_cells {
+        return first ? side_cells{face(0) ? face(0) + j0 * d.f[0].s0 : nullptr, d.f[0].s0, d.f[0].s1} : side_cells{c0 - sx, sy, sz};
+    };
+    const auto right_cells = [&]() -> side_cells {
+        return last ? side_cells{face(1) ? face(1) + j0 * d.f[1].s0 : nullptr, d.f[1].s0, d.f[1].s1} : side_cells{c0 + V * sx, sy, sz};
+    };
+    const side_cells side = need_left ? left_cells() : need_right ? right_cells() : side_cells{nullptr, 0, 0};
+
+    extern __shared__ __align__(16) char shared[];
+    char* const mine = shared + threadIdx.x * 16;
+    char* const beside = shared + (R + 2) * ring<T>::wide + threadIdx.x * sizeof(T);
+    const uint32_t mine_at = (uint32_t)__cvta_generic_to_shared(mine), beside_at = (uint32_t)__cvta_generic_to_shared(beside);
+    const auto copy_cells = [&](uint32_t at, const T* p, int stride, bool valid) {
+        if constexpr (IN_PACKED) copy_async<16>(at, valid ? p : in, valid);
+        else
+        {
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                copy_async<(int)sizeof(T)>(at + v * (int)sizeof(T), valid && v < m ? p + v * stride : in, valid && v < m);
+        }
+    };
+    const auto issue = [&](int k, uint32_t st) { // plane k into the ring at byte st
+        if (k <= k1)
+        {
+            if (k >= 0 && k < nz)
+            {
+                const T* q = c0 + k * sz;
+#pragma unroll
+                for (int r = 0; r < R; ++r) copy_cells(mine_at + st + (r + 1) * ring<T>::wide, q + r * sy, sx, true);
+                if (k >= k0 && k < k1)
+                {
+                    copy_cells(mine_at + st, lo + k * lo_z, lo_x, lo != nullptr);
+                    copy_cells(mine_at + st + (R + 1) * ring<T>::wide, hi + k * hi_z, hi_x, hi != nullptr);
+                    if (need_left || need_right)
+                    {
+#pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            copy_async<(int)sizeof(T)>(beside_at + st + r * ring<T>::narrow, side.p ? side.p + (r * side.y + k * side.z) : in, side.p != nullptr);
+                    }
+                    if (need_both)
+                    {
+                        const side_cells s = right_cells();
+#pragma unroll
+                        for (int r = 0; r < R; ++r)
+                            copy_async<(int)sizeof(T)>(beside_at + st + (R + r) * ring<T>::narrow, s.p ? s.p + (r * s.y + k * s.z) : in, s.p != nullptr);
+                    }
+                }
+            }
+            else
+            {
+                const int f = k < 0 ? 4 : 5, s0 = d.f[f].s0, s1 = d.f[f].s1;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    copy_cells(mine_at + st + (r + 1) * ring<T>::wide, face(f) + (i0 * s0 + (j0 + r) * s1), s0, face(f) != nullptr);
+            }
+        }
+        copy_commit();
+    };
+    const auto wide = [&](uint32_t st, int row) { // row -1 .. R of a plane
+        cells<T> c = *reinterpret_cast<const cells<T>*>(mine + st + (row + 1) * ring<T>::wide);
+        if constexpr (TWICE)
+        {
+#pragma unroll
+            for (int v = 0; v < V; ++v) c.v[v] = mul_rn(T(2), c.v[v]);
+        }
+        return c;
+    };
+    const auto narrow = [&](uint32_t st, int q) {
+        const T v = *reinterpret_cast<const T*>(beside + st + q * ring<T>::narrow);
+        return TWICE ? mul_rn(T(2), v) : v;
+    };
+    // what the exchange's adjoint adds for an image whose neighbour has gradient g: the transposed
+    // update of a zero cell
+    const auto image = [&](T g) { return add_rn(T(0), mul_rn(alpha, add_rn(g, T(0)))); };
+
+    cells<T> below[R], cur[R], next[R];
+#pragma unroll
+    for (int p = 0; p < k_stages; ++p) issue(k0 - 1 + p, p * ring<T>::stage);
+    copy_wait<k_stages - 2>();
+#pragma unroll
+    for (int r = 0; r < R; ++r) below[r] = wide(0, r), cur[r] = wide(ring<T>::stage, r);
+    uint32_t here = ring<T>::stage, free_at = 0; // plane k, the plane before it
+    T* o = out + (i0 * (OUT_PACKED ? 1 : d.osx) + j0 * d.osy + k0 * d.osz);
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k)
+    {
+        issue(k + k_stages - 1, free_at);
+        copy_wait<k_stages - 2>(); // plane k + 1 has landed
+        const uint32_t up = here + ring<T>::stage == ring<T>::bytes ? 0 : here + ring<T>::stage;
+#pragma unroll
+        for (int r = 0; r < R; ++r) next[r] = wide(up, r);
+        const cells<T> clo = wide(here, -1), chi = wide(here, R);
+        // In the transpose a cell beyond a face is not a neighbour (zero) but beside an image of
+        // the cell on this side.
+        const bool bottom = ADJOINT && k == 0, top = ADJOINT && k == nz - 1;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+            T l = __shfl_up_sync(0xffffffffu, cur[r].v[V - 1], 1), e = __shfl_down_sync(0xffffffffu, cur[r].v[0], 1);
+            const T n = narrow(here, r);
+            if (need_left) l = n;
+            else if (need_right) e = n;
+            if (need_both) e = narrow(here, R + r);
+            const T before = ADJOINT && first ? T(0) : l, after = ADJOINT && last ? T(0) : e;
+            cells<T> y;
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+            {
+                const T* x = cur[r].v;
+                T s = add_rn(v > 0 ? x[v > 0 ? v - 1 : 0] : before, v < V - 1 && v < m - 1 ? x[v + 1 < V ? v + 1 : v] : after);
+                s = add_rn(s, r > 0 ? cur[r > 0 ? r - 1 : 0].v[v] : ADJOINT && front ? T(0) : clo.v[v]);
+                s = add_rn(s, r < R - 1 ? cur[r + 1 < R ? r + 1 : r].v[v] : ADJOINT && back ? T(0) : chi.v[v]);
+                s = add_rn(s, bottom ? T(0) : below[r].v[v]);
+                s = add_rn(s, top ? T(0) : next[r].v[v]);
+                y.v[v] = update(x[v], s, alpha);
+            }
+            if constexpr (ADJOINT)
+            {
+                // the face of each axis that a cell of this row touches (an axis has at least two
+                // cells, so at most one), by the order in which its image is added (7: none)
+                const bool edge_y = (r == 0 && front) || (r == R - 1 && back);
+                if (edge_y || bottom || top)
+                {
+                    const auto rank = [&](bool at, int f) { return at ? (int)(d.ranks >> (3 * f)) & 7 : 7; };
+                    const int rl = rank(first, 0), rr = rank(last, 1);
+                    const int ry = r == 0 && front ? rank(true, 2) : rank(r == R - 1 && back, 3);
+                    const int rz = bottom ? rank(true, 4) : rank(top, 5);
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                    {
+                        int rx = 7;
+                        T gx = T(0);
+                        if (v == 0 && rl < 7) rx = rl, gx = l;
+                        if (v == m - 1 && rr < 7) rx = rr, gx = e;
+                        const T gy = r == 0 && front ? T(clo.v[v]) : T(chi.v[v]), gz = bottom ? T(below[r].v[v]) : T(next[r].v[v]);
+                        const T ix = image(gx), iy = image(gy), iz = image(gz);
+                        T a = y.v[v];
+                        // three rounds: the image of the least rank left
+                        const bool x0 = rx < ry && rx < rz, y0 = !x0 && ry < rz;
+                        const int r0 = x0 ? rx : y0 ? ry : rz, lowest = r0;
+                        a = r0 < 7 ? add_rn(a, x0 ? T(ix) : y0 ? T(iy) : T(iz)) : a;
+                        const int sx1 = rx == lowest ? 7 : rx, sy1 = ry == lowest ? 7 : ry, sz1 = rz == lowest ? 7 : rz;
+                        const bool x1 = sx1 < sy1 && sx1 < sz1, y1 = !x1 && sy1 < sz1;
+                        const int r1 = x1 ? sx1 : y1 ? sy1 : sz1;
+                        a = r1 < 7 ? add_rn(a, x1 ? T(ix) : y1 ? T(iy) : T(iz)) : a;
+                        const bool x2 = sx1 < 7 && sx1 != r1, y2 = sy1 < 7 && sy1 != r1, z2 = sz1 < 7 && sz1 != r1;
+                        y.v[v] = x2 || y2 || z2 ? add_rn(a, x2 ? T(ix) : y2 ? T(iy) : T(iz)) : a;
+                    }
+                }
+                else
+                {
+                    if (first && face(0)) y.v[0] = add_rn(y.v[0], image(l));
+                    if (last && face(1))
+                    {
+#pragma unroll
+                        for (int v = 0; v < V; ++v)
+                            if (v == m - 1) y.v[v] = add_rn(y.v[v], image(e));
+                    }
+                }
+            }
+            if (!live) continue;
+            if constexpr (OUT_PACKED)
+                *reinterpret_cast<cells<T>*>(o + r * d.osy) = y;
+            else
+            {
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+                    if (v < m) o[v * d.osx + r * d.osy] = y.v[v];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) below[r] = cur[r], cur[r] = next[r];
+        free_at = here, here = up;
+        o += d.osz;
+    }
+}
+
+// The number of slabs a pass cuts the z axis into: the least time in planes (every slab starts
+// with three loads that nothing hides) over the waves of resident blocks.
+int slabs_of(uint64_t groups, int nz)
+{
+    int best = 1;
+    double least = 0;
+    for (int s = 1; s <= std::max(1, nz / k_min_slab); ++s)
+    {
+        const double blocks = (double)(groups * s), resident = 148.0 * k_resident;
+        const double waves = blocks <= resident ? 1.0 : (double)(int64_t)((blocks + resident - 1) / resident);
+        const double planes = waves * ((nz + s - 1) / s + 3);
+        if (s == 1 || planes < least) best = s, least = planes;
+    }
+    return best;
+}
+
+template <typename T, bool ADJOINT, bool TWICE, bool IN_PACKED, bool OUT_PACKED>
+cudaError_t launch_pass(const ghexb_program_s& P, const void* const* fields, const void* source, void* const* fields_out,
+    void* packed_out, double alpha, cudaStream_t stream)
+{
+    const int n = (int)P.domains.size();
+    const int64_t es = sizeof(T), h = P.halo;
+    const auto in_stride = [&](const program_domain& d, int a) { return IN_PACKED ? (a == 0 ? 1 : a == 1 ? d.row : d.plane) : d.s[a]; };
+    const auto in_cell = [&](int slot) { // interior cell (0, 0, 0)
+        const program_domain& d = P.domains[slot];
+        return IN_PACKED ? static_cast<const char*>(source) + d.offset * es
+                         : static_cast<const char*>(fields[slot]) + h * (d.s[0] + d.s[1] + d.s[2]) * es;
+    };
+    for (int b0 = 0; b0 < n; b0 += k_batch)
+    {
+        pass_args args;
+        args.n = std::min(k_batch, n - b0);
+        uint64_t groups = 0, blocks = 0;
+        int nz = 1;
+        for (int i = 0; i < args.n; ++i)
+        {
+            const program_domain& d = P.domains[b0 + i];
+            const uint64_t chunks = (d.n[0] + cells<T>::V - 1) / cells<T>::V;
+            groups += (chunks * ((d.n[1] + k_rows - 1) / k_rows) + k_threads - 1) / k_threads;
+            nz = std::max(nz, d.n[2]);
+        }
+        const int slabs = slabs_of(groups, nz);
+        for (int i = 0; i < args.n; ++i)
+        {
+            const program_domain& d = P.domains[b0 + i];
+            pass_domain& a = args.d[i];
+            a.in = in_cell(b0 + i);
+            a.out = OUT_PACKED ? static_cast<char*>(packed_out) + d.offset * es
+                               : static_cast<char*>(fields_out[b0 + i]) + h * (d.s[0] + d.s[1] + d.s[2]) * es;
+            a.nx = d.n[0], a.ny = d.n[1], a.nz = d.n[2], a.halo = P.halo;
+            a.isx = (int32_t)in_stride(d, 0), a.isy = (int32_t)in_stride(d, 1), a.isz = (int32_t)in_stride(d, 2);
+            a.osx = (int32_t)(OUT_PACKED ? 1 : d.s[0]), a.osy = (int32_t)(OUT_PACKED ? d.row : d.s[1]);
+            a.osz = (int32_t)(OUT_PACKED ? d.plane : d.s[2]);
+            a.ranks = d.ranks, a.images = d.images;
+            for (int f = 0; f < 6; ++f)
+            {
+                const int axis = f / 2, u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;
+                const int e = ADJOINT ? d.to[f] : d.from[f];
+                a.f[f] = {nullptr, 0, 0};
+                if (e >= 0)
+                {
+                    // the face cell of the neighbour that faces this domain
+                    const program_domain& nb = P.domains[e];
+                    const int64_t at = f % 2 == 0 ? nb.n[axis] - 1 : 0;
+                    a.f[f] = {in_cell(e) + at * in_stride(nb, axis) * es, (int32_t)in_stride(nb, u), (int32_t)in_stride(nb, v)};
+                }
+                else if (!ADJOINT && !IN_PACKED)
+                {
+                    // no exchange fills this halo: the caller's own halo cells (zero after a step)
+                    const int64_t at = f % 2 == 0 ? -1 : d.n[axis];
+                    a.f[f] = {in_cell(b0 + i) + at * d.s[axis] * es, (int32_t)d.s[u], (int32_t)d.s[v]};
+                }
+            }
+            a.chunks = (uint32_t)((d.n[0] + cells<T>::V - 1) / cells<T>::V);
+            a.columns = a.chunks * (uint32_t)((d.n[1] + k_rows - 1) / k_rows);
+            a.groups = (a.columns + k_threads - 1) / k_threads;
+            a.slab = (uint32_t)((d.n[2] + slabs - 1) / slabs);
+            const uint64_t marches = (uint64_t)a.groups * ((d.n[2] + a.slab - 1) / a.slab);
+            const uint64_t all = (uint64_t)(d.n[0] + 2 * h) * (d.n[1] + 2 * h) * (d.n[2] + 2 * h);
+            const uint64_t inner = (uint64_t)d.n[0] * d.n[1] * d.n[2], per = (uint64_t)k_threads * k_halo_cells;
+            a.block0 = (uint32_t)blocks, a.marches = (uint32_t)marches;
+            blocks += marches + (OUT_PACKED ? 0 : (all - inner + per - 1) / per);
+        }
+        if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+        const auto kernel = pass_kernel<T, ADJOINT, TWICE, IN_PACKED, OUT_PACKED>;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring<T>::bytes);
+        if (e != cudaSuccess) return e;
+        kernel<<<(unsigned)blocks, k_threads, ring<T>::bytes, stream>>>(args, (T)alpha);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+template <typename T, bool ADJOINT, bool TWICE>
+cudaError_t launch_passes_t(const ghexb_program_s& P, const void* const* fields, const void* source, void* const* out, void* a,
+    void* b, int steps, double alpha, cudaStream_t stream)
+{
+    // the first pass reads the source as it is given, the later ones a packed buffer, unscaled
+    cudaError_t e = cudaSuccess;
+    for (int s = 0; s < steps && e == cudaSuccess; ++s)
+    {
+        void* dst = source == a ? b : a;
+        const bool packed = source != nullptr, end = out && s == steps - 1;
+        if (s == 0)
+        {
+            if (!packed)
+            {
+                if constexpr (!TWICE)
+                    e = end ? launch_pass<T, ADJOINT, false, false, false>(P, fields, nullptr, out, nullptr, alpha, stream)
+                            : launch_pass<T, ADJOINT, false, false, true>(P, fields, nullptr, nullptr, dst, alpha, stream);
+                else
+                    e = cudaErrorInvalidValue;
+            }
+            else
+                e = end ? launch_pass<T, ADJOINT, TWICE, true, false>(P, nullptr, source, out, nullptr, alpha, stream)
+                        : launch_pass<T, ADJOINT, TWICE, true, true>(P, nullptr, source, nullptr, dst, alpha, stream);
+        }
+        else
+            e = end ? launch_pass<T, ADJOINT, false, true, false>(P, nullptr, source, out, nullptr, alpha, stream)
+                    : launch_pass<T, ADJOINT, false, true, true>(P, nullptr, source, nullptr, dst, alpha, stream);
+        source = dst;
+    }
+    return e;
+}
+
+template <typename T>
+cudaError_t launch_passes_any(const ghexb_program_s& P, const void* const* fields, const void* source, void* const* out, void* a,
+    void* b, int steps, double alpha, bool adjoint, bool twice, cudaStream_t stream)
+{
+    if (!adjoint) return twice ? cudaErrorInvalidValue : launch_passes_t<T, false, false>(P, fields, source, out, a, b, steps, alpha, stream);
+    return twice ? launch_passes_t<T, true, true>(P, fields, source, out, a, b, steps, alpha, stream)
+                 : launch_passes_t<T, true, false>(P, fields, source, out, a, b, steps, alpha, stream);
+}
+} // namespace
+
+cudaError_t launch_passes(const ghexb_program_s& P, const void* const* fields, const void* source, void* const* out, void* a,
+    void* b, int steps, double alpha, bool adjoint, bool twice, cudaStream_t stream)
+{
+    return P.f64 ? launch_passes_any<double>(P, fields, source, out, a, b, steps, alpha, adjoint, twice, stream)
+                 : launch_passes_any<float>(P, fields, source, out, a, b, steps, alpha, adjoint, twice, stream);
+}
+
+// ---- geometry ----------------------------------------------------------------------------------
+void build_program(ghexb_program_s& P, const ghexb_field* fields, int nfields, int halo)
+{
+    const auto require = [](bool ok, const char* why) {
+        if (!ok) throw error(GHEXB_ERR_INVALID, std::string("the program cannot be fused: ") + why);
+    };
+    require(halo >= 1, "the 7-point update needs a halo of width >= 1");
+    const int n = nfields;
+    P.f64 = fields[0]->dtype == GHEXB_F64;
+    P.halo = halo;
+    P.domains.assign(n, program_domain{});
+    P.packed_elements = 0;
+    const int64_t es = fields[0]->esize;
+    // field slots by pattern and domain: the k-th field of a domain pairs with the k-th of its neighbours
+    std::map<std::pair<const ghexb_pattern_s*, int>, std::vector<int>> slots;
+    std::vector<const ghexb_pattern_s*> patterns;
+    for (int s = 0; s < n; ++s)
+    {
+        const auto& f = *fields[s];
+        require(f.pattern->kind == pattern_kind::regular && f.pattern->dim == 3 && f.ndim == 3 && f.num_components == 1, "fields of three regular dimensions only");
+        require((f.dtype == GHEXB_F64 || f.dtype == GHEXB_F32) && f.dtype == fields[0]->dtype, "fields of one floating type only");
+        if (std::find(patterns.begin(), patterns.end(), f.pattern) == patterns.end()) patterns.push_back(f.pattern);
+        slots[{f.pattern, f.domain_index}].push_back(s);
+        program_domain& d = P.domains[s];
+        const auto& dom = f.pattern->domains[f.domain_index];
+        int64_t span = 1, whole = 1;
+        for (int a = 0; a < 3; ++a)
+        {
+            d.n[a] = dom.last[a] - dom.first[a] + 1;
+            require(f.offsets[a] == halo && f.extents[a] == d.n[a] + 2 * halo, "fields padded by the halo on every side only");
+            require(f.byte_strides[a] > 0 && f.byte_strides[a] % es == 0, "strides of whole elements only");
+            d.s[a] = f.byte_strides[a] / es;
+            span += (int64_t)(f.extents[a] + 2 * k_rows) * d.s[a];
+            whole *= f.extents[a];
+        }
+        require(span < (int64_t(1) << 31) && whole < (int64_t(1) << 31), "a field of 2^31 elements");
+        require(d.n[0] >= 2 && d.n[1] >= k_rows && d.n[2] >= 2, "a domain one cell thick, or of fewer rows than a strip");
+        const int64_t unit = 32 / es;
+        d.row = (d.n[0] + unit - 1) / unit * unit;
+        d.plane = d.row * d.n[1];
+        require(d.plane * d.n[2] < (int64_t(1) << 31), "a field of 2^31 elements");
+        d.offset = P.packed_elements;
+        P.packed_elements += (d.plane * d.n[2] + 127) / 128 * 128;
+        for (int k = 0; k < 6; ++k) d.from[k] = d.to[k] = -1;
+        d.ranks = 0777777u; // 7 in every place
+        d.images = 0;
+    }
+    std::vector<int> images_added(n, 0);
+    for (const auto* pattern : patterns)
+        for (int di = 0; di < (int)pattern->domains.size(); ++di)
+        {
+            const auto it = slots.find({pattern, di});
+            if (it == slots.end()) continue;
+            for (const auto& entry : pattern->domains[di].recv)
+            {
+                const auto sit = slots.find({pattern, entry.neighbor});
+                require(sit != slots.end() && sit->second.size() == it->second.size(), "a neighbour without the field");
+                const auto& sources = sit->second;
+                for (size_t k = 0; k < it->second.size(); ++k)
+                {
+                    const int slot = it->second[k], src = sources[k];
+                    program_domain& d = P.domains[slot];
+                    program_domain& o = P.domains[src];
+                    const auto& owner = pattern->domains[entry.neighbor];
+                    for (const auto& sp : entry.spaces)
+                    {
+                        int side[3], outside = 0, face = -1, region = 0;
+                        for (int a = 0, w = 1; a < 3; ++a, w *= 3)
+                        {
+                            const int lo = sp.lfirst[a], hi = sp.llast[a];
+                            side[a] = lo == -halo && hi == -1 ? 0 : lo == 0 && hi == d.n[a] - 1 ? 1 : lo == d.n[a] && hi == d.n[a] + halo - 1 ? 2 : -1;
+                            require(side[a] >= 0, "a halo region that several domains fill, or of another width than the update's halo");
+                            region += w * side[a];
+                            if (side[a] != 1) ++outside, face = 2 * a + (side[a] == 2);
+                        }
+                        require(outside > 0 && !((d.images >> region) & 1u), "a halo region that is filled twice");
+                        d.images |= 1u << region;
+                        if (outside != 1) continue; // edges and corners: no cell of the update reads them
+                        for (int a = 0; a < 3; ++a)
+                        {
+                            const int at = sp.has_src ? sp.sfirst[a] : sp.gfirst[a] - owner.first[a];
+                            const int want = side[a] == 1 ? 0 : side[a] == 0 ? o.n[a] - halo : 0;
+                            require(at == want && (side[a] != 1 || o.n[a] == d.n[a]), "a face that is part of its neighbour's face");
+                        }
+                        require(d.s[0] > 0 && o.to[face ^ 1] < 0, "a face with two images");
+                        d.from[face] = src;
+                        o.to[face ^ 1] = slot;
+                        o.ranks = (o.ranks & ~(7u << (3 * (face ^ 1)))) | (uint32_t)images_added[src]++ << (3 * (face ^ 1));
+                    }
+                }
+            }
+        }
+}
+
+// ---- sum of squares of the interiors -------------------------------------------------------------
+namespace
+{
+constexpr int k_sum_threads = 256, k_sum_chunks = 8; // a block adds 2048 chunks of 16 bytes
+struct sum_args
+{
+    struct
+    {
+        const void* p;
+        int32_t nx, ny, nz;
+        uint32_t chunks, block0;
+        int64_t sx, sy, sz;
+        fast_div by_chunks, by_rows; // of chunks and ny, for arrays of fewer than 2^31 chunks
+    } d[k_batch];
+    int n;
+};
+
+__device__ __forceinline__ double block_sum(double v)
+{
+    __shared__ double part[32];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = threadIdx.x < blockDim.x >> 5 ? part[threadIdx.x] : 0.0;
+    if (threadIdx.x < 32)
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v; // of thread 0
+}
+
+// One pass over the interiors, in order of memory: bound by HBM (or L2 where the fields fit it).
+template <typename T, bool PACKED>
+__global__ void __launch_bounds__(k_sum_threads) sumsq_kernel(const __grid_constant__ sum_args args, double* __restrict__ partials)
+{
+    constexpr int V = cells<T>::V;
+    uint32_t b = blockIdx.x;
+    int di = 0;
+    while (di + 1 < args.n && b >= args.d[di + 1].block0) ++di;
+    const auto& d = args.d[di];
+    b -= d.block0;
+    const uint64_t all = (uint64_t)d.chunks * d.ny * d.nz;
+    const T* __restrict__ p = static_cast<const T*>(d.p);
+    cells<T> c[k_sum_chunks];
+    int m[k_sum_chunks];
+#pragma unroll
+    for (int q = 0; q < k_sum_chunks; ++q)
+    {
+        const uint64_t e = ((uint64_t)b * k_sum_chunks + q) * k_sum_threads + threadIdx.x;
+        m[q] = 0;
+        if (e >= all) continue;
+        const uint32_t row = all >> 31 ? (uint32_t)(e / d.chunks) : d.by_chunks.div((uint32_t)e), i0 = (uint32_t)(e - (uint64_t)row * d.chunks) * V;
+        const uint32_t k = d.by_rows.div(row), j = row - k * d.ny;
+        m[q] = min(V, d.nx - (int)i0);
+        if constexpr (PACKED)
+        {
+            union
+            {
+                int4 w;
+                cells<T> c;
+            } u;
+            u.w = __ldg(reinterpret_cast<const int4*>(p + (i0 + j * d.sy + k * d.sz)));
+            c[q] = u.c;
+        }
+        else
+        {
+#pragma unroll
+            for (int v = 0; v < V; ++v) c[q].v[v] = v < m[q] ? __ldg(p + ((int64_t)(i0 + v) * d.sx + j * d.sy + k * d.sz)) : T(0);
+        }
+    }
+    double s = 0;
+#pragma unroll
+    for (int q = 0; q < k_sum_chunks; ++q)
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (v < m[q]) s = __dadd_rn(s, __dmul_rn((double)c[q].v[v], (double)c[q].v[v]));
+    s = block_sum(s);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+}
+
+template <typename T> __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* __restrict__ partials, uint32_t n, T* out)
+{
+    double s = 0;
+    for (uint32_t i = threadIdx.x; i < n; i += 1024) s = __dadd_rn(s, partials[i]);
+    s = block_sum(s);
+    if (threadIdx.x == 0) *out = (T)s;
+}
+
+struct grad_args
+{
+    struct
+    {
+        const void* p;
+        void* out;
+        int32_t ex, ey, ez;
+        uint32_t block0;
+        int64_t sx, sy, sz;
+        fast_div by_row, by_rows; // of ex and ey, for arrays of fewer than 2^31 cells
+    } d[k_batch];
+    int n, halo;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(k_sum_threads) sumsq_grad_kernel(const __grid_constant__ grad_args args, const T* __restrict__ g)
+{
+    uint32_t b = blockIdx.x;
+    int di = 0;
+    while (di + 1 < args.n && b >= args.d[di + 1].block0) ++di;
+    const auto& d = args.d[di];
+    b -= d.block0;
+    const int h = args.halo;
+    const uint64_t all = (uint64_t)d.ex * d.ey * d.ez;
+    const T scale = __ldg(g);
+    const T* __restrict__ p = static_cast<const T*>(d.p);
+    T* __restrict__ out = static_cast<T*>(d.out);
+    T x[k_sum_chunks];
+    int64_t at[k_sum_chunks];
+#pragma unroll
+    for (int q = 0; q < k_sum_chunks; ++q)
+    {
+        const uint64_t e = ((uint64_t)b * k_sum_chunks + q) * k_sum_threads + threadIdx.x;
+        at[q] = -1;
+        x[q] = T(0);
+        if (e >= all) continue;
+        const uint32_t row = all >> 31 ? (uint32_t)(e / d.ex) : d.by_row.div((uint32_t)e);
+        const int i = (int)(e - (uint64_t)row * d.ex), k = (int)d.by_rows.div(row), j = (int)(row - (uint32_t)k * d.ey);
+        at[q] = (int64_t)i * d.sx + (int64_t)j * d.sy + (int64_t)k * d.sz;
+        if (i >= h && i < d.ex - h && j >= h && j < d.ey - h && k >= h && k < d.ez - h)
+            x[q] = mul_rn(scale, mul_rn(T(2), __ldg(p + at[q])));
+    }
+#pragma unroll
+    for (int q = 0; q < k_sum_chunks; ++q)
+        if (at[q] >= 0) out[at[q]] = x[q];
+}
+
+uint64_t sum_blocks(int V, const int32_t* n)
+{
+    const uint64_t chunks = (uint64_t)((n[0] + V - 1) / V) * n[1] * n[2], per = (uint64_t)k_sum_threads * k_sum_chunks;
+    return (chunks + per - 1) / per;
+}
+
+template <typename T>
+cudaError_t launch_sumsq_t(const interior* d, int n, bool packed, double* partials, void* out, cudaStream_t stream)
+{
+    uint64_t done = 0;
+    for (int b0 = 0; b0 < n; b0 += k_batch)
+    {
+        sum_args args;
+        args.n = std::min(k_batch, n - b0);
+        uint64_t blocks = 0;
+        for (int i = 0; i < args.n; ++i)
+        {
+            const interior& s = d[b0 + i];
+            auto& a = args.d[i];
+            a.p = s.p, a.nx = s.n[0], a.ny = s.n[1], a.nz = s.n[2], a.sx = s.s[0], a.sy = s.s[1], a.sz = s.s[2];
+            a.chunks = (uint32_t)((s.n[0] + cells<T>::V - 1) / cells<T>::V);
+            a.by_chunks = fast_div::make(a.chunks), a.by_rows = fast_div::make((uint32_t)s.n[1]);
+            a.block0 = (uint32_t)blocks;
+            blocks += sum_blocks(cells<T>::V, s.n);
+        }
+        if (done + blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+        if (packed) sumsq_kernel<T, true><<<(unsigned)blocks, k_sum_threads, 0, stream>>>(args, partials + done);
+        else
+            sumsq_kernel<T, false><<<(unsigned)blocks, k_sum_threads, 0, stream>>>(args, partials + done);
+        done += blocks;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    sum_partials_kernel<T><<<1, 1024, 0, stream>>>(partials, (uint32_t)done, static_cast<T*>(out));
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_grad_t(const interior* d, void* const* out, int n, int halo, const void* g, cudaStream_t stream)
+{
+    for (int b0 = 0; b0 < n; b0 += k_batch)
+    {
+        grad_args args;
+        args.n = std::min(k_batch, n - b0), args.halo = halo;
+        uint64_t blocks = 0;
+        const uint64_t per = (uint64_t)k_sum_threads * k_sum_chunks;
+        for (int i = 0; i < args.n; ++i)
+        {
+            const interior& s = d[b0 + i];
+            auto& a = args.d[i];
+            a.p = s.p, a.out = out[b0 + i], a.ex = s.n[0], a.ey = s.n[1], a.ez = s.n[2], a.sx = s.s[0], a.sy = s.s[1], a.sz = s.s[2];
+            a.by_row = fast_div::make((uint32_t)s.n[0]), a.by_rows = fast_div::make((uint32_t)s.n[1]);
+            a.block0 = (uint32_t)blocks;
+            blocks += ((uint64_t)s.n[0] * s.n[1] * s.n[2] + per - 1) / per;
+        }
+        if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+        sumsq_grad_kernel<T><<<(unsigned)blocks, k_sum_threads, 0, stream>>>(args, static_cast<const T*>(g));
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+} // namespace
+
+int64_t sumsq_blocks(bool f64, const int32_t (*extents)[3], int n)
+{
+    uint64_t blocks = 0;
+    for (int i = 0; i < n; ++i) blocks += sum_blocks(f64 ? cells<double>::V : cells<float>::V, extents[i]);
+    return (int64_t)blocks;
+}
+
+cudaError_t launch_sumsq(bool f64, const interior* d, int n, bool packed, double* partials, void* out, cudaStream_t stream)
+{
+    return f64 ? launch_sumsq_t<double>(d, n, packed, partials, out, stream) : launch_sumsq_t<float>(d, n, packed, partials, out, stream);
+}
+
+cudaError_t launch_sumsq_grad(bool f64, const interior* d, void* const* out, int n, int halo, const void* g, cudaStream_t stream)
+{
+    return f64 ? launch_grad_t<double>(d, out, n, halo, g, stream) : launch_grad_t<float>(d, out, n, halo, g, stream);
+}
+} // namespace ghexb

@@ -52,6 +52,7 @@ typedef struct ghexb_field_s* ghexb_field; /* a field bound to a pattern: GHEX's
 typedef struct ghexb_co_s* ghexb_co;
 typedef struct ghexb_handle_s* ghexb_handle;
 typedef struct ghexb_plan_s* ghexb_plan;
+typedef struct ghexb_program_s* ghexb_program;
 
 typedef struct ghexb_plan_info_t
 {
@@ -380,6 +381,37 @@ int ghexb_calibrate_rows(const void* src, void* dst, int64_t rows, int n, int64_
  * round-to-nearest in a fixed order without fused multiply-adds. */
 int ghexb_stencil7(int dtype, int n, const void* const* in, void* const* out, const int64_t* extents,
                    const int64_t* strides, int halo, double alpha, int adjoint, void* stream);
+
+/* ---- the program itself (exchange, then update, `steps` times) and its transpose, one kernel a
+ * step. No counterpart in GHEX. A program is the geometry of one exchange: 3-D regular fields of
+ * one type (GHEXB_F32 or GHEXB_F64), padded by `halo` on every side, every face of a domain facing
+ * one whole face of one neighbour or nothing; any other exchange is refused with
+ * GHEXB_ERR_INVALID. The fields' memory is not kept. */
+int ghexb_program_create(const ghexb_field* fields, int n, int halo, ghexb_program* out);
+int ghexb_program_destroy(ghexb_program program);
+/* Size of a packed buffer (16-byte aligned device memory) that holds every interior. */
+int ghexb_program_buffer_bytes(ghexb_program program, int64_t* bytes);
+/* `steps` >= 1 passes. The first reads the caller's fields (fields[i] laid out as the i-th field
+ * of ghexb_program_create) or, with fields == NULL, the packed buffer `source`. Each pass but the
+ * last writes the packed buffer of `a` and `b` that it does not read (a first); the last writes
+ * out[i] in the caller's layout or, with out == NULL, a packed buffer too. adjoint == 0: a pass is
+ * the exchange and the update, with the output halo 0. adjoint != 0: a pass is the update's
+ * transpose and the exchange's adjoint. twice != 0 (adjoint, from `source`): the source times two,
+ * the gradient of its sum of squares. Results have the bits of ghexb_plan_launch and
+ * ghexb_stencil7 (or of the latter's transpose and ghexb_plan_adjoint_launch) in turn. */
+int ghexb_program_steps(ghexb_program program, const void* const* fields, const void* source, void* const* out, void* a,
+                        void* b, int steps, double alpha, int adjoint, int twice, void* stream);
+/* Sum of squares of the interiors of n 3-D arrays (arguments as ghexb_stencil7's), added in 64
+ * bits in a fixed order, into *out (device, of the arrays' type). `partials` is device memory for
+ * as many doubles as ghexb_sumsq_partials says. ghexb_program_sumsq: the same sum, bit for bit, of
+ * a program's packed buffer. ghexb_sumsq_grad: out = *g * (2 in) on the interiors, 0 on the halos
+ * (g on the device). */
+int ghexb_sumsq_partials(int dtype, int n, const int64_t* extents, int halo, int64_t* count);
+int ghexb_sumsq(int dtype, int n, const void* const* in, const int64_t* extents, const int64_t* strides, int halo,
+                double* partials, int64_t count, void* out, void* stream);
+int ghexb_program_sumsq(ghexb_program program, const void* source, double* partials, int64_t count, void* out, void* stream);
+int ghexb_sumsq_grad(int dtype, int n, const void* const* in, void* const* out, const int64_t* extents,
+                     const int64_t* strides, int halo, const void* g, void* stream);
 
 #ifdef __cplusplus
 }

@@ -1,0 +1,145 @@
+"""The program in fused passes (ghexb_program_*) against the exchange and the update run one after
+the other, bit for bit: final fields, exchanged inputs, gradients, and the graphed loss and
+gradient. The cases are where a pass can go wrong: rows that end inside a 16-byte chunk, strips and
+slabs that overlap, domains two cells thick, one domain along an axis (its own neighbour), axes that
+are not periodic (the halo keeps its values and its gradient), uneven domains, a halo of width 2,
+more domains than one launch takes. Every value is one of the same operations with the same
+roundings, so the tolerance is zero."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from ghex_b200 import autograd as AG
+from ghex_b200 import workloads as W
+
+from gpu_helpers import RegularRun, bits_equal
+
+pytestmark = pytest.mark.gpu
+
+ALPHA = 0.1
+
+
+def make(cuda, shape, parts, periodic, halo, dtype, seed):
+    w = W.RegularWorkload("program", shape, periodic, W.regular_decomposition(shape, parts, seed))
+    w.fields = [W.FieldSpec("x", dtype, (halo,) * 6, 3)]
+    run = RegularRun(w, cuda)
+    dx = AG.DifferentiableExchange(run.ctx, run.bis)
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    xs = [torch.empty_like(t).uniform_(-1, 1, generator=gen) for t in run.dev["x"]]  # halos too
+    return dx, xs
+
+
+def separately(dx, xs, steps, halo):
+    first = None
+    for _ in range(steps):
+        xs = dx(*xs)
+        first = first or xs
+        xs = AG.stencil7(xs, ALPHA, halo)
+    return first, xs
+
+
+def equal(a, b):
+    torch.cuda.synchronize()
+    return sum(bits_equal(x.detach().cpu().numpy(), y.detach().cpu().numpy()) for x, y in zip(a, b)) == 0
+
+
+CASES = [
+    ((16, 12, 10), (2, 2, 2), (True, True, True), 1, None),
+    ((9, 11, 7), (2, 2, 2), (True, True, True), 1, None),
+    ((4, 4, 4), (2, 2, 2), (True, True, True), 1, None),
+    ((37, 29, 41), (3, 2, 2), (True, False, True), 1, 4),
+    ((70, 33, 26), (2, 3, 1), (False, False, False), 1, 9),
+    ((131, 10, 50), (1, 2, 2), (True, True, False), 1, None),
+    ((24, 18, 20), (2, 2, 2), (True, False, True), 2, None),
+    ((24, 20, 12), (4, 3, 3), (True, True, True), 1, None),
+    ((300, 40, 9), (2, 2, 1), (True, True, True), 1, 2),
+]
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shape,parts,periodic,halo,seed", CASES)
+def test_fused_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
+    dx, x0 = make(cuda, shape, parts, periodic, halo, dtype, seed)
+    assert dx._program(halo) is not None
+    for steps in (1, 2, 3):
+        grads, fields, ins = [], [], []
+        for fused in (False, True):
+            leaves = [x.clone().requires_grad_(True) for x in x0]
+            xs = [x.clone() for x in leaves]
+            if fused:
+                ys = AG.diffusion_program(dx, xs, steps, ALPHA, halo)
+                first = xs
+            else:
+                first, ys = separately(dx, xs, steps, halo)
+            weights = [torch.linspace(-1, 1, y.numel(), dtype=y.dtype, device=cuda).reshape(y.shape) for y in ys]
+            loss = sum((y * v).sum() for y, v in zip(ys, weights))
+            grads.append(torch.autograd.grad(loss, leaves, retain_graph=True))
+            fields.append(ys)
+            ins.append(first)
+            # the exchanged inputs used as well
+            loss = loss + sum((x * v).sum() for x, v in zip(first, weights))
+            grads[-1] += torch.autograd.grad(loss, leaves)
+        assert equal(*fields)
+        assert equal(*ins)
+        assert equal(*grads)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shape,parts,periodic,halo,seed", CASES[:1] + CASES[3:6])
+def test_graphed_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
+    """Inputs of the fields' layout (read in place) and of another one (copied), and the loss
+    against a sum in 64 bits: n squares added in 64 bits err by less than n roundings."""
+    dx, x0 = make(cuda, shape, parts, periodic, halo, dtype, seed)
+    for steps in (1, 4):
+        graphed = AG.GraphedDiffusion(dx, x0, steps, ALPHA, halo)
+        for scale, relaid in ((1.0, False), (-0.5, True)):
+            xs = [x * scale for x in x0]
+            leaves = [x.clone().requires_grad_(True) for x in xs]
+            _, ys = separately(dx, [x.clone() for x in leaves], steps, halo)
+            loss = AG.interior_loss(ys, halo)
+            grads = torch.autograd.grad(loss, leaves)
+            got, g = graphed.run([x.contiguous() for x in xs] if relaid else xs)
+            assert equal([got], [loss])
+            assert equal(g, grads)
+            h = halo
+            exact = sum((y.detach().double()[h:-h, h:-h, h:-h] ** 2).sum() for y in ys)
+            n = sum(y.numel() for y in ys)
+            eps = torch.finfo(loss.dtype).eps
+            assert abs(loss.double() - exact) <= (n * torch.finfo(torch.float64).eps + eps) * exact
+
+
+def test_interior_loss_is_differentiable_twice(cuda):
+    """A gradient of the loss that is differentiated in turn: d/dx sum((dL/dx)^2) = 8 x."""
+    x = torch.randn((6, 5, 7), dtype=torch.float64, device=cuda, requires_grad=True)
+    (g,) = torch.autograd.grad(AG.interior_loss([x]), [x], create_graph=True)
+    (gg,) = torch.autograd.grad((g ** 2).sum(), [x])
+    expected = torch.zeros_like(x)
+    expected[1:-1, 1:-1, 1:-1] = 8 * x.detach()[1:-1, 1:-1, 1:-1]
+    assert bits_equal(gg.cpu().numpy(), expected.cpu().numpy()) == 0
+
+
+@pytest.mark.parametrize("case", ["halo", "thin", "fields of two types"])
+def test_other_exchanges_run_unfused(cuda, case):
+    """A pattern halo wider than the update's, domains one cell thick, fields of two types: the
+    program is not fused, and is what it was."""
+    if case == "halo":
+        dx, xs = make(cuda, (12, 12, 12), (2, 2, 2), (True, True, True), 2, np.float64, None)
+        assert dx._program(1) is None
+        _, ref = separately(dx, [x.clone() for x in xs], 2, 1)
+        assert equal(AG.diffusion_program(dx, [x.clone() for x in xs], 2, ALPHA, 1), ref)
+    elif case == "thin":
+        dx, xs = make(cuda, (8, 8, 2), (2, 2, 2), (True, True, True), 1, np.float64, None)
+        assert dx._program(1) is None
+        _, ref = separately(dx, [x.clone() for x in xs], 2, 1)
+        assert equal(AG.diffusion_program(dx, [x.clone() for x in xs], 2, ALPHA, 1), ref)
+    else:
+        shape = (8, 8, 8)
+        w = W.RegularWorkload("two", shape, (True,) * 3, W.regular_decomposition(shape, (2, 2, 2)))
+        w.fields = [W.FieldSpec("a", np.float64, (1,) * 6, 3), W.FieldSpec("b", np.float32, (1,) * 6, 4)]
+        run = RegularRun(w, cuda)
+        dx = AG.DifferentiableExchange(run.ctx, run.bis)
+        assert dx._program(1) is None
+        with pytest.raises(TypeError, match="one dtype"):
+            AG.diffusion_program(dx, run.dev["a"] + run.dev["b"], 2, ALPHA)
