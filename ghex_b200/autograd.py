@@ -244,6 +244,12 @@ class _Program:
         call("ghexb_program_steps", self._h, array(fields), address(source), array(out), address(a), address(b), steps,
              float(alpha), int(adjoint), int(twice), C.c_void_p(stream.cuda_stream))
 
+    def status(self) -> int:
+        """The passes' status word since the last call (0: every load arrived in time)."""
+        v = C.c_uint()
+        call("ghexb_program_status", self._h, C.byref(v))
+        return v.value
+
     def __del__(self, _release=_capi.release):
         _release("ghexb_program_destroy", getattr(self, "_h", None))
         self._h = None

@@ -1059,7 +1059,18 @@ int ghexb_program_create(const ghexb_field* fields, int n, int halo, ghexb_progr
         for (int i = 0; i < n; ++i) require(fields[i] != nullptr, "null field handle");
         auto p = std::make_unique<ghexb_program_s>();
         ghexb::build_program(*p, fields, n, halo);
+        ghexb::check_cuda(cudaMalloc(&p->status, sizeof(unsigned)), "cudaMalloc(program status)");
+        ghexb::check_cuda(cudaMemset(p->status, 0, sizeof(unsigned)), "cudaMemset(program status)");
         *out = p.release();
+    });
+}
+
+int ghexb_program_status(ghexb_program program, unsigned* status)
+{
+    return guarded([&] {
+        require(program && status, "null argument");
+        ghexb::check_cuda(cudaMemcpy(status, program->status, sizeof(unsigned), cudaMemcpyDeviceToHost), "cudaMemcpy(program status)");
+        ghexb::check_cuda(cudaMemset(program->status, 0, sizeof(unsigned)), "cudaMemset(program status)");
     });
 }
 

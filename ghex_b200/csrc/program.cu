@@ -11,10 +11,12 @@
 // The fields between two passes are the program's own, and packed: interiors only, rows on
 // 32-byte boundaries, so that a thread moves 16 bytes at a time whatever the domains' extents.
 //
-// One step on 8 domains of 128 x 128 x 64, as exchange + update kernels and as a pass: forward
-// 6.6 + 42.3 us and 27.9 us in float64, 5.5 + 31.2 us and 13.7 us in float32; transposed 8.6 +
-// 42.9 us and 43.3 us, 7.9 + 28.1 us and 23.4 us. The floor, one read and one write of every cell
-// at the HBM rate, is 20.5 and 10.2 us.
+// One step on 8 domains of 128 x 128 x 64, in us: exchange kernel + update kernel, a pass, and the
+// floor (one read and one write of every cell at the HBM rate; the float32 fields fit the L2):
+//   forward     float64  6.6 + 42.3   22.8   20.5     float32  5.5 + 31.2   11.7   10.2
+//   transposed  float64  8.6 + 42.9   32.5   20.5     float32  7.9 + 28.1   18.1   10.2
+// and on 12 uneven domains of 500 x 510 x 250 in all, float64: forward 32.1 + 261.8, 182.8, 155.7;
+// transposed 37.8 + 262.8, 206.9, 155.7.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,7 +24,9 @@
 #include <string>
 #include <utility>
 
+#include "async_copy.hpp"
 #include "program.hpp"
+#include "staged.hpp"
 
 namespace ghexb
 {
@@ -50,6 +54,72 @@ template <typename T> struct alignas(16) cells
     static constexpr int V = 16 / (int)sizeof(T);
     T v[V];
 };
+
+// Cell by cell. Sums of float cells two at a time (add.f32x2: the same rounding); products stay
+// scalar, since a packed product is contracted with the sum that follows it, explicit roundings or
+// not (of 2^20 random mul.rn.f32x2 + add.rn.f32x2 all had the bits of the fused form).
+__device__ __forceinline__ float2 add_rn(float2 a, float2 b)
+{
+    float2 c;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(c.x), "=f"(c.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return c;
+}
+template <typename T> __device__ __forceinline__ cells<T> add_rn(const cells<T>& a, const cells<T>& b)
+{
+    cells<T> c;
+    if constexpr (sizeof(T) == 4)
+    {
+#pragma unroll
+        for (int v = 0; v < cells<T>::V; v += 2)
+        {
+            const float2 s = add_rn(make_float2(a.v[v], a.v[v + 1]), make_float2(b.v[v], b.v[v + 1]));
+            c.v[v] = s.x, c.v[v + 1] = s.y;
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int v = 0; v < cells<T>::V; ++v) c.v[v] = add_rn(a.v[v], b.v[v]);
+    }
+    return c;
+}
+template <typename T> __device__ __forceinline__ cells<T> mul_rn(T f, const cells<T>& a)
+{
+    cells<T> c;
+#pragma unroll
+    for (int v = 0; v < cells<T>::V; ++v) c.v[v] = mul_rn(f, a.v[v]);
+    return c;
+}
+// The update of a row's cells x (m of them count) between the cells l and e and the rows around:
+// s - 6 x is taken as s + (-6) x, the same value.
+template <typename T>
+__device__ __forceinline__ cells<T> update(const cells<T>& x, T l, T e, int m, const cells<T>& up, const cells<T>& down, const cells<T>& below,
+    const cells<T>& above, T alpha)
+{
+    constexpr int V = cells<T>::V;
+    cells<T> s;
+#pragma unroll
+    for (int v = 0; v < V; ++v) s.v[v] = add_rn(v > 0 ? x.v[v > 0 ? v - 1 : 0] : l, v < V - 1 && v < m - 1 ? x.v[v + 1 < V ? v + 1 : v] : e);
+    s = add_rn(s, up);
+    s = add_rn(s, down);
+    s = add_rn(s, below);
+    s = add_rn(s, above);
+    return add_rn(x, mul_rn(alpha, add_rn(s, mul_rn(T(-6), x))));
+}
+template <typename T> __device__ __forceinline__ void zero(cells<T>& a)
+{
+#pragma unroll
+    for (int v = 0; v < cells<T>::V; ++v) a.v[v] = T(0);
+}
+template <typename T> __device__ __forceinline__ cells<T> zero_if(bool z, const cells<T>& a)
+{
+    cells<T> c;
+#pragma unroll
+    for (int v = 0; v < cells<T>::V; ++v) c.v[v] = z ? T(0) : a.v[v];
+    return c;
+}
 
 constexpr int k_batch = 32; // domains per launch
 
@@ -105,7 +175,7 @@ template <int N> __device__ __forceinline__ void copy_async(uint32_t dst, const 
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <typename T, bool ADJOINT, bool TWICE>
+template <typename T, bool ADJOINT, bool TWICE, int THREADS>
 __device__ __forceinline__ void write_halo(const pass_domain& d, T alpha, uint32_t block)
 {
     const int h = d.halo, nx = d.nx, ny = d.ny, nz = d.nz;
@@ -115,7 +185,7 @@ __device__ __forceinline__ void write_halo(const pass_domain& d, T alpha, uint32
     T* __restrict__ out = static_cast<T*>(d.out);
     for (int q = 0; q < k_halo_cells; ++q)
     {
-        uint32_t c = (block * k_halo_cells + q) * k_threads + threadIdx.x;
+        uint32_t c = (block * k_halo_cells + q) * THREADS + threadIdx.x;
         int i, j, k;
         if (c < zcells)
         {
@@ -161,7 +231,87 @@ __device__ __forceinline__ void write_halo(const pass_domain& d, T alpha, uint32
     }
 }
 
-template <typename T, bool ADJOINT, bool TWICE, bool IN_PACKED, bool OUT_PACKED>
+// What the exchange's adjoint adds for an image whose neighbour has gradient g: the transposed
+// update of a zero cell.
+template <typename T> __device__ __forceinline__ T image(T g, T alpha) { return add_rn(T(0), mul_rn(alpha, add_rn(g, T(0)))); }
+
+// The images of a row of cells along x and y alone: those of its cells along y (`along`: the row is
+// on face y- or y+), and along x of its first cell (fi) or of the last that counts (la); *_first:
+// that one comes before the one along y.
+template <typename T>
+__device__ __forceinline__ void add_row_images(cells<T>& y, bool along, const cells<T>& iy, bool fi, bool la, T il, T ie, bool fi_first, bool la_first,
+    int m)
+{
+#pragma unroll
+    for (int v = 0; v < cells<T>::V; ++v)
+    {
+        const bool at_l = v == 0 && fi, at_e = v == m - 1 && la;
+        const T ix = at_l ? il : ie;
+        const bool x_first = at_l ? fi_first : la_first;
+        const T before = add_rn(y.v[v], ix); // the image along x first
+        T a = (at_l || at_e) && x_first ? before : y.v[v];
+        const T with = add_rn(a, T(iy.v[v]));
+        a = along ? with : a;
+        const T after = add_rn(a, ix);
+        y.v[v] = (at_l || at_e) && !x_first ? after : a;
+    }
+}
+
+// Adds to a row of cells the images of the faces that it touches (fr, ba: y-, y+; fi, la: x-, x+;
+// bo, to: z-, z+): l, e, across, beyond are the cells beyond along x, y and z. An axis has at least two cells, so a
+// cell touches at most one face of each; their images are added in the order of their ranks (7:
+// no image).
+template <typename T>
+__device__ __forceinline__ void add_images(cells<T>& y, const pass_domain& d, bool fr, bool ba, bool fi, bool la, bool bo, bool to, int m, T l, T e,
+    const cells<T>& across, const cells<T>& beyond, T alpha)
+{
+    constexpr int V = cells<T>::V;
+    if (!(fr || ba || bo || to))
+    {
+        if (fi && d.f[0].p) y.v[0] = add_rn(y.v[0], image(l, alpha));
+        if (la && d.f[1].p)
+        {
+            const T add = image(e, alpha);
+            if (m == V) y.v[V - 1] = add_rn(y.v[V - 1], add);
+            else
+            {
+#pragma unroll
+                for (int v = 0; v < V - 1; ++v)
+                {
+                    const T sum = add_rn(y.v[v], add);
+                    y.v[v] = v == m - 1 ? sum : y.v[v];
+                }
+            }
+        }
+        return;
+    }
+    const auto rank = [&](bool at, int f) { return at ? (int)(d.ranks >> (3 * f)) & 7 : 7; };
+    const int rl = rank(fi, 0), rr = rank(la, 1);
+    const int ry = fr ? rank(true, 2) : rank(ba, 3);
+    const int rz = bo ? rank(true, 4) : rank(to, 5);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+    {
+        int rx = 7;
+        T gx = T(0);
+        if (v == 0 && rl < 7) rx = rl, gx = l;
+        if (v == m - 1 && rr < 7) rx = rr, gx = e;
+        const T ix = image(gx, alpha), iy = image(across.v[v], alpha), iz = image(beyond.v[v], alpha);
+        T a = y.v[v];
+        // three rounds: the image of the least rank left
+        const bool x0 = rx < ry && rx < rz, y0 = !x0 && ry < rz;
+        const int r0 = x0 ? rx : y0 ? ry : rz;
+        a = r0 < 7 ? add_rn(a, x0 ? T(ix) : y0 ? T(iy) : T(iz)) : a;
+        const int x1 = rx == r0 ? 7 : rx, y1 = ry == r0 ? 7 : ry, z1 = rz == r0 ? 7 : rz;
+        const bool xs = x1 < y1 && x1 < z1, ys = !xs && y1 < z1;
+        const int r1 = xs ? x1 : ys ? y1 : z1;
+        a = r1 < 7 ? add_rn(a, xs ? T(ix) : ys ? T(iy) : T(iz)) : a;
+        const bool x2 = x1 < 7 && x1 != r1, y2 = y1 < 7 && y1 != r1, z2 = z1 < 7 && z1 != r1;
+        y.v[v] = x2 || y2 || z2 ? add_rn(a, x2 ? T(ix) : y2 ? T(iy) : T(iz)) : a;
+    }
+}
+
+template <typename T, bool ADJOINT, bool OUT_PACKED>
 __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __grid_constant__ pass_args args, T alpha)
 {
     constexpr int V = cells<T>::V, R = k_rows;
@@ -172,7 +322,7 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
     b -= d.block0;
     if (b >= d.marches)
     {
-        if constexpr (!OUT_PACKED) write_halo<T, ADJOINT, TWICE>(d, alpha, b - d.marches);
+        if constexpr (!OUT_PACKED) write_halo<T, ADJOINT, false, k_threads>(d, alpha, b - d.marches);
         return;
     }
     const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -184,7 +334,7 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
     const int j0 = min((int)strip * R, ny - R); // the last strip overlaps the one before (same values)
     const T* __restrict__ in = static_cast<const T*>(d.in);
     T* __restrict__ out = static_cast<T*>(d.out);
-    const int sx = IN_PACKED ? 1 : d.isx, sy = d.isy, sz = d.isz;
+    const int sx = d.isx, sy = d.isy, sz = d.isz;
     const bool first = i0 == 0, last = i0 + V >= nx; // the chunk touches face x-, x+
     const int lane = threadIdx.x & 31;
 
@@ -218,13 +368,9 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
     char* const beside = shared + (R + 2) * ring<T>::wide + threadIdx.x * sizeof(T);
     const uint32_t mine_at = (uint32_t)__cvta_generic_to_shared(mine), beside_at = (uint32_t)__cvta_generic_to_shared(beside);
     const auto copy_cells = [&](uint32_t at, const T* p, int stride, bool valid) {
-        if constexpr (IN_PACKED) copy_async<16>(at, valid ? p : in, valid);
-        else
-        {
 #pragma unroll
-            for (int v = 0; v < V; ++v)
-                copy_async<(int)sizeof(T)>(at + v * (int)sizeof(T), valid && v < m ? p + v * stride : in, valid && v < m);
-        }
+        for (int v = 0; v < V; ++v)
+            copy_async<(int)sizeof(T)>(at + v * (int)sizeof(T), valid && v < m ? p + v * stride : in, valid && v < m);
     };
     const auto issue = [&](int k, uint32_t st) { // plane k into the ring at byte st
         if (k <= k1)
@@ -264,21 +410,11 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
         copy_commit();
     };
     const auto wide = [&](uint32_t st, int row) { // row -1 .. R of a plane
-        cells<T> c = *reinterpret_cast<const cells<T>*>(mine + st + (row + 1) * ring<T>::wide);
-        if constexpr (TWICE)
-        {
-#pragma unroll
-            for (int v = 0; v < V; ++v) c.v[v] = mul_rn(T(2), c.v[v]);
-        }
-        return c;
+        return *reinterpret_cast<const cells<T>*>(mine + st + (row + 1) * ring<T>::wide);
     };
     const auto narrow = [&](uint32_t st, int q) {
-        const T v = *reinterpret_cast<const T*>(beside + st + q * ring<T>::narrow);
-        return TWICE ? mul_rn(T(2), v) : v;
+        return *reinterpret_cast<const T*>(beside + st + q * ring<T>::narrow);
     };
-    // what the exchange's adjoint adds for an image whose neighbour has gradient g: the transposed
-    // update of a zero cell
-    const auto image = [&](T g) { return add_rn(T(0), mul_rn(alpha, add_rn(g, T(0)))); };
 
     cells<T> below[R], cur[R], next[R];
 #pragma unroll
@@ -309,62 +445,10 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
             else if (need_right) e = n;
             if (need_both) e = narrow(here, R + r);
             const T before = ADJOINT && first ? T(0) : l, after = ADJOINT && last ? T(0) : e;
-            cells<T> y;
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-            {
-                const T* x = cur[r].v;
-                T s = add_rn(v > 0 ? x[v > 0 ? v - 1 : 0] : before, v < V - 1 && v < m - 1 ? x[v + 1 < V ? v + 1 : v] : after);
-                s = add_rn(s, r > 0 ? cur[r > 0 ? r - 1 : 0].v[v] : ADJOINT && front ? T(0) : clo.v[v]);
-                s = add_rn(s, r < R - 1 ? cur[r + 1 < R ? r + 1 : r].v[v] : ADJOINT && back ? T(0) : chi.v[v]);
-                s = add_rn(s, bottom ? T(0) : below[r].v[v]);
-                s = add_rn(s, top ? T(0) : next[r].v[v]);
-                y.v[v] = update(x[v], s, alpha);
-            }
+            cells<T> y = update(cur[r], before, after, m, r > 0 ? cur[r > 0 ? r - 1 : 0] : zero_if(ADJOINT && front, clo),
+                r < R - 1 ? cur[r + 1 < R ? r + 1 : r] : zero_if(ADJOINT && back, chi), zero_if(bottom, below[r]), zero_if(top, next[r]), alpha);
             if constexpr (ADJOINT)
-            {
-                // the face of each axis that a cell of this row touches (an axis has at least two
-                // cells, so at most one), by the order in which its image is added (7: none)
-                const bool edge_y = (r == 0 && front) || (r == R - 1 && back);
-                if (edge_y || bottom || top)
-                {
-                    const auto rank = [&](bool at, int f) { return at ? (int)(d.ranks >> (3 * f)) & 7 : 7; };
-                    const int rl = rank(first, 0), rr = rank(last, 1);
-                    const int ry = r == 0 && front ? rank(true, 2) : rank(r == R - 1 && back, 3);
-                    const int rz = bottom ? rank(true, 4) : rank(top, 5);
-#pragma unroll
-                    for (int v = 0; v < V; ++v)
-                    {
-                        int rx = 7;
-                        T gx = T(0);
-                        if (v == 0 && rl < 7) rx = rl, gx = l;
-                        if (v == m - 1 && rr < 7) rx = rr, gx = e;
-                        const T gy = r == 0 && front ? T(clo.v[v]) : T(chi.v[v]), gz = bottom ? T(below[r].v[v]) : T(next[r].v[v]);
-                        const T ix = image(gx), iy = image(gy), iz = image(gz);
-                        T a = y.v[v];
-                        // three rounds: the image of the least rank left
-                        const bool x0 = rx < ry && rx < rz, y0 = !x0 && ry < rz;
-                        const int r0 = x0 ? rx : y0 ? ry : rz, lowest = r0;
-                        a = r0 < 7 ? add_rn(a, x0 ? T(ix) : y0 ? T(iy) : T(iz)) : a;
-                        const int sx1 = rx == lowest ? 7 : rx, sy1 = ry == lowest ? 7 : ry, sz1 = rz == lowest ? 7 : rz;
-                        const bool x1 = sx1 < sy1 && sx1 < sz1, y1 = !x1 && sy1 < sz1;
-                        const int r1 = x1 ? sx1 : y1 ? sy1 : sz1;
-                        a = r1 < 7 ? add_rn(a, x1 ? T(ix) : y1 ? T(iy) : T(iz)) : a;
-                        const bool x2 = sx1 < 7 && sx1 != r1, y2 = sy1 < 7 && sy1 != r1, z2 = sz1 < 7 && sz1 != r1;
-                        y.v[v] = x2 || y2 || z2 ? add_rn(a, x2 ? T(ix) : y2 ? T(iy) : T(iz)) : a;
-                    }
-                }
-                else
-                {
-                    if (first && face(0)) y.v[0] = add_rn(y.v[0], image(l));
-                    if (last && face(1))
-                    {
-#pragma unroll
-                        for (int v = 0; v < V; ++v)
-                            if (v == m - 1) y.v[v] = add_rn(y.v[v], image(e));
-                    }
-                }
-            }
+                add_images<T>(y, d, r == 0 && front, r == R - 1 && back, first, last, bottom, top, m, l, e, r == 0 && front ? clo : chi, bottom ? below[r] : next[r], alpha);
             if (!live) continue;
             if constexpr (OUT_PACKED)
                 *reinterpret_cast<cells<T>*>(o + r * d.osy) = y;
@@ -382,15 +466,274 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
     }
 }
 
+// ---- packed input: tiles through the copy engine -------------------------------------------------
+// A pass over a packed buffer reads a tile of rows (with the rows and chunks around it) per plane
+// by one tensor-map load into a ring of k_tile_stages planes, issued by a warp of its own as the
+// other warps release stages; cells beyond the domain arrive as zeros. The rows beyond faces y- and
+// y+ come beside the tile by one bulk load each, the plane beyond z- or z+ through the neighbour's
+// map, and the cells beyond x- and x+ by single element copies of the threads that need them. A
+// thread marches along z with its column of 16 bytes by R rows, as above, and reads each plane of
+// it once from shared memory; the load/store unit moves no byte into shared memory, which is what
+// bounded the thread-private rings above on packed input (L1 82 % busy; a step of 27.9 / 43.3 us in
+// float64, 13.7 / 23.4 us in float32, 215 / 314 us on the large grid).
+//
+// What bounds it now: forward, HBM (float64) and the latency of a plane's chain of roundings with
+// 16 warps per SM (float32); the transpose, its images: a tile on a face adds them after the sum, a
+// second chain of roundings. Measured alike or slower: 128 or 224 marching threads, 2 or 3 rows a
+// thread (24.4 / 36.2 us), 5 or 6 planes, a block barrier in place of the released stages (25 / 37).
+constexpr int k_tile_threads = 96, k_tile_stages = 4, k_tile_resident = 4; // marching threads, planes, blocks per SM
+constexpr int k_tile_rows = 4; // rows of a thread; 2 for domains of fewer rows
+
+struct tile_domain
+{
+    pass_domain d;
+    uint32_t cw, strips;  // chunks and strips of a tile
+    uint32_t xtiles, ytiles;
+    uint32_t pitch;       // bytes of a tile row: cw + 2 chunks
+    uint32_t face0, side0, stage; // byte offsets in a stage of the face rows and the cells beside, and its size
+};
+struct tile_args
+{
+    tile_domain t[k_batch];
+    CUtensorMap map[k_batch][3]; // the domain's buffer, the ones of its neighbours across z- and z+
+    int32_t zlo[k_batch], zhi[k_batch]; // the plane of those next to the domain, or -1 and nz of its own (zeros)
+    unsigned* status;
+    int n;
+};
+
+__device__ __forceinline__ void load_tile(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+template <typename T, bool ADJOINT, bool TWICE, bool OUT_PACKED, int R>
+__global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_kernel(const __grid_constant__ tile_args args, T alpha)
+{
+    constexpr int V = cells<T>::V, S = k_tile_stages;
+    uint32_t b = blockIdx.x;
+    int di = 0;
+    while (di + 1 < args.n && b >= args.t[di + 1].d.block0) ++di;
+    const tile_domain& g = args.t[di];
+    const pass_domain& d = g.d;
+    b -= d.block0;
+    if (b >= d.marches)
+    {
+        if constexpr (!OUT_PACKED) write_halo<T, ADJOINT, TWICE, k_tile_threads + 32>(d, alpha, b - d.marches);
+        return;
+    }
+    const int nx = d.nx, ny = d.ny, nz = d.nz;
+    const uint32_t tx = b % g.xtiles, rest = b / g.xtiles, ty = rest % g.ytiles, bz = rest / g.ytiles;
+    const int k0 = (int)(bz * d.slab), k1 = min(nz, k0 + (int)d.slab);
+    const int h = (int)g.strips * R;
+    const int c0 = (int)min(tx * g.cw, d.chunks - g.cw), y0 = min((int)ty * h, max(0, ny - h)); // the last tiles overlap
+    const uint32_t columns = g.cw * g.strips, column = min((uint32_t)threadIdx.x, columns - 1);
+    const bool live = threadIdx.x < columns;
+    const int s = (int)(column / g.cw), c = (int)(column - (uint32_t)s * g.cw);
+    const int i0 = (c0 + c) * V, m = min(V, nx - i0), j0 = min(y0 + s * R, ny - R);
+    const bool first = i0 == 0, last = i0 + V >= nx, front = j0 == 0, back = j0 + R == ny;
+    const auto face = [&](int f) { return static_cast<const T*>(d.f[f].p); };
+
+    extern __shared__ __align__(128) unsigned char dynamic[];
+    unsigned char* const shared = dynamic + (128u - smem_u32(dynamic) % 128u) % 128u; // stages start on 128 bytes
+    __shared__ __align__(8) uint64_t full[S], empty[S]; // a stage has landed; every warp has read it
+    if (threadIdx.x == 0)
+    {
+#pragma unroll
+        for (int q = 0; q < S; ++q) mbar_init(&full[q], 1), mbar_init(&empty[q], k_tile_threads / 32);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    // planes k0 - 1 .. k1 of the slab, numbered from 0
+    const int planes = k1 - k0 + 2;
+    const bool row_lo = y0 == 0 && face(2), row_hi = y0 + h >= ny && face(3);
+    const bool edge_tile = row_lo || row_hi || (c0 == 0 && face(0)) || ((uint32_t)c0 + g.cw >= d.chunks && face(1)); // it touches a face with images
+    const uint32_t wide = g.cw * 16u;
+    const auto issue = [&](int q, int st) { // the loads of plane q into stage st
+        const int k = k0 - 1 + q;
+        unsigned char* dst = shared + (uint32_t)st * g.stage;
+        const bool inner = q > 0 && q + 1 < planes;
+        mbar_expect_tx(&full[st], g.pitch * (uint32_t)(h + 2) + (inner ? wide * ((row_lo ? 1u : 0u) + (row_hi ? 1u : 0u)) : 0u));
+        const int which = k < 0 ? 1 : k == nz ? 2 : 0;
+        load_tile(dst, &args.map[di][which], c0 * V - V, y0 - 1, which == 0 ? k : which == 1 ? args.zlo[di] : args.zhi[di], &full[st]);
+        if (inner && row_lo) bulk_load(dst + g.face0, face(2) + (c0 * V + k * d.f[2].s1), wide, &full[st]);
+        if (inner && row_hi) bulk_load(dst + g.face0 + wide, face(3) + (c0 * V + k * d.f[3].s1), wide, &full[st]);
+    };
+    if (threadIdx.x >= k_tile_threads) // the last warp issues the loads, as stages become free
+    {
+        if (threadIdx.x == k_tile_threads)
+        {
+            bool ok = true;
+            for (int q = 0; q < planes && ok; ++q)
+            {
+                const int st = q % S;
+                ok = q < S || mbar_wait(&empty[st], (uint32_t)(q / S - 1) & 1u);
+                if (ok) issue(q, st);
+                else atomicOr(args.status, 1u);
+            }
+            // the block's shared memory is not given back before its last loads have landed (the
+            // other threads wait for every plane; this is for those that gave up)
+            for (int q = max(0, planes - S); q < planes && ok; ++q) ok = mbar_wait(&full[q % S], (uint32_t)(q / S) & 1u);
+        }
+        return;
+    }
+    // the cells beyond x- and x+ beside this thread's rows
+    const bool side_lo = first && face(0), side_hi = last && face(1);
+    const uint32_t side = g.side0 + (uint32_t)(s * R) * (uint32_t)sizeof(T), side_other = side + (uint32_t)h * (uint32_t)sizeof(T);
+    const auto issue_sides = [&](int q, int st) {
+        if ((side_lo || side_hi) && q > 0 && q + 1 < planes)
+        {
+            const uint32_t at = smem_u32(shared + (uint32_t)st * g.stage);
+            const int k = k0 - 1 + q;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+            {
+                if (side_lo) copy_async<(int)sizeof(T)>(at + side + r * (int)sizeof(T), face(0) + ((j0 + r) * d.f[0].s0 + k * d.f[0].s1), true);
+                if (side_hi) copy_async<(int)sizeof(T)>(at + side_other + r * (int)sizeof(T), face(1) + ((j0 + r) * d.f[1].s0 + k * d.f[1].s1), true);
+            }
+        }
+        copy_commit();
+    };
+    bool failed = false; // a load did not arrive in time: nothing more is waited for or stored
+    const auto wait = [&](int st, uint32_t parity) {
+        if (!failed && !mbar_wait(&full[st], parity))
+        {
+            failed = true;
+            atomicOr(args.status, 1u);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < S; ++q) issue_sides(q, q);
+    const uint32_t at = (uint32_t)(j0 - y0 + 1) * g.pitch + (uint32_t)(c + 1) * 16u; // row 0 of the strip in a stage
+    const auto read = [&](uint32_t off) {
+        cells<T> v = *reinterpret_cast<const cells<T>*>(shared + off);
+        if constexpr (TWICE)
+        {
+#pragma unroll
+            for (int e = 0; e < V; ++e) v.v[e] = mul_rn(T(2), v.v[e]);
+        }
+        return v;
+    };
+    const auto read_one = [&](uint32_t off) {
+        const T v = *reinterpret_cast<const T*>(shared + off);
+        return TWICE ? mul_rn(T(2), v) : v;
+    };
+    // the rows before and after the strip and the cells beside it in a stage: the tile's own (zeros
+    // beyond the domain) or, forward, what came from beyond a face
+    const bool far_lo = front && row_lo, far_hi = back && row_hi;
+    const uint32_t face_lo = g.face0 + (uint32_t)c * 16u, face_hi = face_lo + wide;
+    const uint32_t lo_at = !ADJOINT && far_lo ? face_lo : at - g.pitch, hi_at = !ADJOINT && far_hi ? face_hi : at + R * g.pitch;
+    const uint32_t left_at = !ADJOINT && side_lo ? side : at - (uint32_t)sizeof(T), left_step = !ADJOINT && side_lo ? (uint32_t)sizeof(T) : g.pitch;
+    const uint32_t right_at = !ADJOINT && side_hi ? side_other : at + 16u, right_step = !ADJOINT && side_hi ? (uint32_t)sizeof(T) : g.pitch;
+
+    cells<T> below[R], cur[R], next[R];
+    wait(0, 0);
+    wait(1, 0);
+#pragma unroll
+    for (int r = 0; r < R; ++r) below[r] = read(at + r * g.pitch), cur[r] = read(g.stage + at + r * g.pitch);
+    // after the warp's reads of a stage. The copy engine's writes do not wait for reads that are
+    // merely issued: in the loop the values read are used (stored) before, here the fence waits.
+    const auto release = [&](int st) {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(&empty[st]);
+    };
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    release(0);
+    int st = 1, up = 2 % S; // the stages of planes k and k + 1
+    uint32_t up_parity = 2 / S;
+    T* o = static_cast<T*>(d.out) + (i0 * (OUT_PACKED ? 1 : d.osx) + j0 * d.osy + k0 * d.osz);
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k)
+    {
+        const int q = k - k0 + 1;
+        issue_sides(q - 1 + S, st == 0 ? S - 1 : st - 1); // (a thread's own, read one plane ago)
+        wait(up, up_parity);
+        copy_wait<S - 1>(); // the sides of plane q
+        const uint32_t here = (uint32_t)st * g.stage, above = (uint32_t)up * g.stage;
+#pragma unroll
+        for (int r = 0; r < R; ++r) next[r] = read(above + at + r * g.pitch);
+        const cells<T> clo = read(here + lo_at), chi = read(here + hi_at);
+        // In the transpose a plane beyond a face is not a neighbour but images of this plane.
+        const bool bottom = ADJOINT && k == 0, top = ADJOINT && k == nz - 1;
+        cells<T> beyond[R];
+        if (ADJOINT && (bottom || top))
+        {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+            {
+                beyond[r] = bottom ? below[r] : next[r];
+                below[r] = zero_if(bottom, below[r]), next[r] = zero_if(top, next[r]);
+            }
+        }
+        cells<T> y[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            y[r] = update(cur[r], read_one(here + left_at + r * left_step), read_one(here + right_at + r * right_step), m,
+                r > 0 ? cur[r > 0 ? r - 1 : 0] : clo, r < R - 1 ? cur[r + 1 < R ? r + 1 : r] : chi, below[r], next[r], alpha);
+        if (ADJOINT && (edge_tile || bottom || top)) // the same for the whole block
+        {
+            // the images of a thread's rows together: their chains of roundings are long, and overlap
+            T l[R], e[R];
+            cells<T> across[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+            {
+                l[r] = side_lo ? read_one(here + side + r * (uint32_t)sizeof(T)) : T(0);
+                e[r] = side_hi ? read_one(here + side_other + r * (uint32_t)sizeof(T)) : T(0);
+                zero(across[r]);
+                if (r == 0 && far_lo) across[r] = read(here + face_lo);
+                if (r == R - 1 && far_hi) across[r] = read(here + face_hi);
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+            {
+                const bool lo = r == 0 && far_lo, hi = r == R - 1 && far_hi;
+                if (bottom || top) add_images<T>(y[r], d, lo, hi, side_lo, side_hi, bottom, top, m, l[r], e[r], across[r], beyond[r], alpha);
+                else
+                {
+                    cells<T> iy;
+#pragma unroll
+                    for (int v = 0; v < V; ++v) iy.v[v] = image(across[r].v[v], alpha);
+                    const uint32_t ry = (d.ranks >> (lo ? 6 : 9)) & 7u;
+                    const bool along = lo || hi;
+                    add_row_images<T>(y[r], along, iy, side_lo, side_hi, image(l[r], alpha), image(e[r], alpha), !along || (d.ranks & 7u) < ry,
+                        !along || ((d.ranks >> 3) & 7u) < ry, m);
+                }
+            }
+        }
+        if (live && !failed)
+        {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if constexpr (OUT_PACKED)
+                    *reinterpret_cast<cells<T>*>(o + r * d.osy) = y[r];
+                else
+                {
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                        if (v < m) o[v * d.osx + r * d.osy] = y[r].v[v];
+                }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) below[r] = cur[r], cur[r] = next[r];
+        o += d.osz;
+        release(st);
+        st = up;
+        if (++up == S) up = 0, up_parity ^= 1u;
+    }
+    copy_wait<0>();
+}
+
 // The number of slabs a pass cuts the z axis into: the least time in planes (every slab starts
-// with three loads that nothing hides) over the waves of resident blocks.
-int slabs_of(uint64_t groups, int nz)
+// with a few loads that nothing hides) over the waves of resident blocks. groups: blocks a slab.
+int slabs_of(uint64_t groups, int nz, int per_sm)
 {
     int best = 1;
     double least = 0;
     for (int s = 1; s <= std::max(1, nz / k_min_slab); ++s)
     {
-        const double blocks = (double)(groups * s), resident = 148.0 * k_resident;
+        const double blocks = (double)(groups * s), resident = 148.0 * per_sm;
         const double waves = blocks <= resident ? 1.0 : (double)(int64_t)((blocks + resident - 1) / resident);
         const double planes = waves * ((nz + s - 1) / s + 3);
         if (s == 1 || planes < least) best = s, least = planes;
@@ -398,18 +741,68 @@ int slabs_of(uint64_t groups, int nz)
     return best;
 }
 
-template <typename T, bool ADJOINT, bool TWICE, bool IN_PACKED, bool OUT_PACKED>
-cudaError_t launch_pass(const ghexb_program_s& P, const void* const* fields, const void* source, void* const* fields_out,
-    void* packed_out, double alpha, cudaStream_t stream)
+// What a pass reads and writes: fields in the caller's layout, or (fields null) a packed buffer.
+struct pass_io
+{
+    const void* const* in;
+    const void* source;
+    void* const* out;
+    void* packed;
+};
+
+int64_t in_stride(const program_domain& d, bool packed, int a) { return packed ? (a == 0 ? 1 : a == 1 ? d.row : d.plane) : d.s[a]; }
+const char* in_cell(const ghexb_program_s& P, const pass_io& io, int slot) // interior cell (0, 0, 0)
+{
+    const program_domain& d = P.domains[slot];
+    const int64_t es = P.f64 ? 8 : 4;
+    return io.source ? static_cast<const char*>(io.source) + d.offset * es
+                     : static_cast<const char*>(io.in[slot]) + P.halo * (d.s[0] + d.s[1] + d.s[2]) * es;
+}
+
+void fill_domain(pass_domain& a, const ghexb_program_s& P, const pass_io& io, int slot, bool adjoint)
+{
+    const program_domain& d = P.domains[slot];
+    const int64_t es = P.f64 ? 8 : 4, h = P.halo;
+    const bool packed = io.source != nullptr;
+    a.in = in_cell(P, io, slot);
+    a.out = io.out ? static_cast<char*>(io.out[slot]) + h * (d.s[0] + d.s[1] + d.s[2]) * es : static_cast<char*>(io.packed) + d.offset * es;
+    a.nx = d.n[0], a.ny = d.n[1], a.nz = d.n[2], a.halo = P.halo;
+    a.isx = (int32_t)in_stride(d, packed, 0), a.isy = (int32_t)in_stride(d, packed, 1), a.isz = (int32_t)in_stride(d, packed, 2);
+    a.osx = (int32_t)(io.out ? d.s[0] : 1), a.osy = (int32_t)(io.out ? d.s[1] : d.row), a.osz = (int32_t)(io.out ? d.s[2] : d.plane);
+    a.ranks = d.ranks, a.images = d.images;
+    for (int f = 0; f < 6; ++f)
+    {
+        const int axis = f / 2, u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;
+        const int e = adjoint ? d.to[f] : d.from[f];
+        a.f[f] = {nullptr, 0, 0};
+        if (e >= 0)
+        {
+            // the face cells of the neighbour that face this domain
+            const program_domain& nb = P.domains[e];
+            const int64_t at = f % 2 == 0 ? nb.n[axis] - 1 : 0;
+            a.f[f] = {in_cell(P, io, e) + at * in_stride(nb, packed, axis) * es, (int32_t)in_stride(nb, packed, u), (int32_t)in_stride(nb, packed, v)};
+        }
+        else if (!adjoint && !packed)
+        {
+            // no exchange fills this halo: the caller's own halo cells (zero after a step)
+            const int64_t at = f % 2 == 0 ? -1 : d.n[axis];
+            a.f[f] = {in_cell(P, io, slot) + at * d.s[axis] * es, (int32_t)d.s[u], (int32_t)d.s[v]};
+        }
+    }
+}
+
+// blocks of `threads` threads that write a domain's halo
+uint64_t halo_blocks(const program_domain& d, int64_t h, int threads)
+{
+    const uint64_t all = (uint64_t)(d.n[0] + 2 * h) * (d.n[1] + 2 * h) * (d.n[2] + 2 * h);
+    const uint64_t inner = (uint64_t)d.n[0] * d.n[1] * d.n[2], per = (uint64_t)threads * k_halo_cells;
+    return (all - inner + per - 1) / per;
+}
+
+template <typename T, bool ADJOINT, bool OUT_PACKED>
+cudaError_t launch_fields(const ghexb_program_s& P, const pass_io& io, double alpha, cudaStream_t stream)
 {
     const int n = (int)P.domains.size();
-    const int64_t es = sizeof(T), h = P.halo;
-    const auto in_stride = [&](const program_domain& d, int a) { return IN_PACKED ? (a == 0 ? 1 : a == 1 ? d.row : d.plane) : d.s[a]; };
-    const auto in_cell = [&](int slot) { // interior cell (0, 0, 0)
-        const program_domain& d = P.domains[slot];
-        return IN_PACKED ? static_cast<const char*>(source) + d.offset * es
-                         : static_cast<const char*>(fields[slot]) + h * (d.s[0] + d.s[1] + d.s[2]) * es;
-    };
     for (int b0 = 0; b0 < n; b0 += k_batch)
     {
         pass_args args;
@@ -419,54 +812,26 @@ cudaError_t launch_pass(const ghexb_program_s& P, const void* const* fields, con
         for (int i = 0; i < args.n; ++i)
         {
             const program_domain& d = P.domains[b0 + i];
-            const uint64_t chunks = (d.n[0] + cells<T>::V - 1) / cells<T>::V;
-            groups += (chunks * ((d.n[1] + k_rows - 1) / k_rows) + k_threads - 1) / k_threads;
-            nz = std::max(nz, d.n[2]);
-        }
-        const int slabs = slabs_of(groups, nz);
-        for (int i = 0; i < args.n; ++i)
-        {
-            const program_domain& d = P.domains[b0 + i];
             pass_domain& a = args.d[i];
-            a.in = in_cell(b0 + i);
-            a.out = OUT_PACKED ? static_cast<char*>(packed_out) + d.offset * es
-                               : static_cast<char*>(fields_out[b0 + i]) + h * (d.s[0] + d.s[1] + d.s[2]) * es;
-            a.nx = d.n[0], a.ny = d.n[1], a.nz = d.n[2], a.halo = P.halo;
-            a.isx = (int32_t)in_stride(d, 0), a.isy = (int32_t)in_stride(d, 1), a.isz = (int32_t)in_stride(d, 2);
-            a.osx = (int32_t)(OUT_PACKED ? 1 : d.s[0]), a.osy = (int32_t)(OUT_PACKED ? d.row : d.s[1]);
-            a.osz = (int32_t)(OUT_PACKED ? d.plane : d.s[2]);
-            a.ranks = d.ranks, a.images = d.images;
-            for (int f = 0; f < 6; ++f)
-            {
-                const int axis = f / 2, u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;
-                const int e = ADJOINT ? d.to[f] : d.from[f];
-                a.f[f] = {nullptr, 0, 0};
-                if (e >= 0)
-                {
-                    // the face cell of the neighbour that faces this domain
-                    const program_domain& nb = P.domains[e];
-                    const int64_t at = f % 2 == 0 ? nb.n[axis] - 1 : 0;
-                    a.f[f] = {in_cell(e) + at * in_stride(nb, axis) * es, (int32_t)in_stride(nb, u), (int32_t)in_stride(nb, v)};
-                }
-                else if (!ADJOINT && !IN_PACKED)
-                {
-                    // no exchange fills this halo: the caller's own halo cells (zero after a step)
-                    const int64_t at = f % 2 == 0 ? -1 : d.n[axis];
-                    a.f[f] = {in_cell(b0 + i) + at * d.s[axis] * es, (int32_t)d.s[u], (int32_t)d.s[v]};
-                }
-            }
+            fill_domain(a, P, io, b0 + i, ADJOINT);
             a.chunks = (uint32_t)((d.n[0] + cells<T>::V - 1) / cells<T>::V);
             a.columns = a.chunks * (uint32_t)((d.n[1] + k_rows - 1) / k_rows);
             a.groups = (a.columns + k_threads - 1) / k_threads;
-            a.slab = (uint32_t)((d.n[2] + slabs - 1) / slabs);
-            const uint64_t marches = (uint64_t)a.groups * ((d.n[2] + a.slab - 1) / a.slab);
-            const uint64_t all = (uint64_t)(d.n[0] + 2 * h) * (d.n[1] + 2 * h) * (d.n[2] + 2 * h);
-            const uint64_t inner = (uint64_t)d.n[0] * d.n[1] * d.n[2], per = (uint64_t)k_threads * k_halo_cells;
-            a.block0 = (uint32_t)blocks, a.marches = (uint32_t)marches;
-            blocks += marches + (OUT_PACKED ? 0 : (all - inner + per - 1) / per);
+            groups += a.groups;
+            nz = std::max(nz, d.n[2]);
+        }
+        const int slabs = slabs_of(groups, nz, k_resident);
+        for (int i = 0; i < args.n; ++i)
+        {
+            pass_domain& a = args.d[i];
+            a.slab = (uint32_t)((a.nz + slabs - 1) / slabs);
+            a.block0 = (uint32_t)blocks;
+            const uint64_t marches = (uint64_t)a.groups * ((a.nz + a.slab - 1) / a.slab);
+            a.marches = (uint32_t)marches;
+            blocks += marches + (OUT_PACKED ? 0 : halo_blocks(P.domains[b0 + i], P.halo, k_threads));
         }
         if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-        const auto kernel = pass_kernel<T, ADJOINT, TWICE, IN_PACKED, OUT_PACKED>;
+        const auto kernel = pass_kernel<T, ADJOINT, OUT_PACKED>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring<T>::bytes);
         if (e != cudaSuccess) return e;
         kernel<<<(unsigned)blocks, k_threads, ring<T>::bytes, stream>>>(args, (T)alpha);
@@ -474,6 +839,102 @@ cudaError_t launch_pass(const ghexb_program_s& P, const void* const* fields, con
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+// The tile of a domain of `chunks` by `strips` columns: the one of least cost, a block's time in
+// units of its threads' work plus the cells its loads move beyond its own.
+void shape_tile(tile_domain& t, uint32_t chunks, uint32_t strips, int V, int rows)
+{
+    double least = 0;
+    t.cw = 0;
+    const uint32_t widest = std::min<uint32_t>(k_tile_threads, 256u / V - 2u); // a load box is at most 256 elements wide
+    const uint32_t few = (chunks + widest - 1) / widest;
+    for (uint32_t nt = few; nt <= std::min(chunks, few + 16); ++nt)
+    {
+        const uint32_t cw = (chunks + nt - 1) / nt;
+        const uint32_t hs = std::min(std::min((uint32_t)k_tile_threads / cw, strips), 64u);
+        const double blocks = (double)((chunks + cw - 1) / cw) * ((strips + hs - 1) / hs);
+        const double cost = blocks * (1.0 + (double)(cw + 2) * (hs * rows + 2) / (k_tile_threads * rows));
+        if (t.cw == 0 || cost < least) t.cw = cw, t.strips = hs, least = cost;
+    }
+    t.xtiles = (chunks + t.cw - 1) / t.cw;
+    t.ytiles = (strips + t.strips - 1) / t.strips;
+}
+
+template <typename T, bool ADJOINT, bool TWICE, bool OUT_PACKED, int R>
+cudaError_t launch_tiles_r(const ghexb_program_s& P, const pass_io& io, double alpha, cudaStream_t stream)
+{
+    const int n = (int)P.domains.size(), V = cells<T>::V;
+    const int64_t es = sizeof(T);
+    for (int b0 = 0; b0 < n; b0 += k_batch)
+    {
+        tile_args args;
+        args.n = std::min(k_batch, n - b0);
+        args.status = P.status;
+        uint64_t groups = 0, blocks = 0;
+        uint32_t stage = 0;
+        int nz = 1;
+        for (int i = 0; i < args.n; ++i)
+        {
+            const program_domain& d = P.domains[b0 + i];
+            tile_domain& t = args.t[i];
+            fill_domain(t.d, P, io, b0 + i, ADJOINT);
+            t.d.chunks = (uint32_t)((d.n[0] + V - 1) / V);
+            shape_tile(t, t.d.chunks, (uint32_t)((d.n[1] + R - 1) / R), V, R);
+            const uint32_t h = t.strips * R;
+            t.pitch = (t.cw + 2) * 16u;
+            t.face0 = (t.pitch * (h + 2) + 15u) / 16u * 16u;
+            t.side0 = t.face0 + 2u * t.cw * 16u;
+            t.stage = (t.side0 + 2u * h * (uint32_t)es + 127u) / 128u * 128u;
+            stage = std::max(stage, t.stage);
+            groups += (uint64_t)t.xtiles * t.ytiles;
+            nz = std::max(nz, d.n[2]);
+            for (int w = 0; w < 3; ++w)
+            {
+                const int e = w == 0 ? -1 : ADJOINT ? d.to[w + 3] : d.from[w + 3];
+                const int slot = e >= 0 ? e : b0 + i; // without a neighbour: beyond the domain's own planes, zeros
+                const program_domain& nb = P.domains[slot];
+                const cuuint64_t dims[3] = {(cuuint64_t)nb.n[0], (cuuint64_t)nb.n[1], (cuuint64_t)nb.n[2]};
+                const cuuint64_t strides[2] = {(cuuint64_t)(nb.row * es), (cuuint64_t)(nb.plane * es)};
+                const cuuint32_t box[3] = {(t.cw + 2) * V, h + 2, 1};
+                if (encode_tensor_map(&args.map[i][w], es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+                        const_cast<char*>(in_cell(P, io, slot)), dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) != CUDA_SUCCESS)
+                    return cudaErrorInvalidValue;
+                if (w == 1) args.zlo[i] = e >= 0 ? nb.n[2] - 1 : -1;
+                if (w == 2) args.zhi[i] = e >= 0 ? 0 : nb.n[2];
+            }
+        }
+        const uint32_t bytes = stage * k_tile_stages + 128u;
+        const int per_sm = std::max(1, std::min(k_tile_resident, (int)(227u * 1024u / (bytes + 1024u))));
+        const int slabs = slabs_of(groups, nz, per_sm);
+        for (int i = 0; i < args.n; ++i)
+        {
+            tile_domain& t = args.t[i];
+            pass_domain& a = t.d;
+            a.slab = (uint32_t)((a.nz + slabs - 1) / slabs);
+            a.block0 = (uint32_t)blocks;
+            const uint64_t marches = (uint64_t)t.xtiles * t.ytiles * ((a.nz + a.slab - 1) / a.slab);
+            a.marches = (uint32_t)marches;
+            blocks += marches + (OUT_PACKED ? 0 : halo_blocks(P.domains[b0 + i], P.halo, k_tile_threads + 32));
+        }
+        if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+        const auto kernel = tile_kernel<T, ADJOINT, TWICE, OUT_PACKED, R>;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+        kernel<<<(unsigned)blocks, k_tile_threads + 32, bytes, stream>>>(args, (T)alpha);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+template <typename T, bool ADJOINT, bool TWICE, bool OUT_PACKED>
+cudaError_t launch_tiles(const ghexb_program_s& P, const pass_io& io, double alpha, cudaStream_t stream)
+{
+    bool rows = true;
+    for (const auto& d : P.domains) rows = rows && d.n[1] >= k_tile_rows;
+    return rows ? launch_tiles_r<T, ADJOINT, TWICE, OUT_PACKED, k_tile_rows>(P, io, alpha, stream)
+                : launch_tiles_r<T, ADJOINT, TWICE, OUT_PACKED, k_rows>(P, io, alpha, stream);
 }
 
 template <typename T, bool ADJOINT, bool TWICE>
@@ -484,26 +945,12 @@ cudaError_t launch_passes_t(const ghexb_program_s& P, const void* const* fields,
     cudaError_t e = cudaSuccess;
     for (int s = 0; s < steps && e == cudaSuccess; ++s)
     {
-        void* dst = source == a ? b : a;
-        const bool packed = source != nullptr, end = out && s == steps - 1;
-        if (s == 0)
-        {
-            if (!packed)
-            {
-                if constexpr (!TWICE)
-                    e = end ? launch_pass<T, ADJOINT, false, false, false>(P, fields, nullptr, out, nullptr, alpha, stream)
-                            : launch_pass<T, ADJOINT, false, false, true>(P, fields, nullptr, nullptr, dst, alpha, stream);
-                else
-                    e = cudaErrorInvalidValue;
-            }
-            else
-                e = end ? launch_pass<T, ADJOINT, TWICE, true, false>(P, nullptr, source, out, nullptr, alpha, stream)
-                        : launch_pass<T, ADJOINT, TWICE, true, true>(P, nullptr, source, nullptr, dst, alpha, stream);
-        }
-        else
-            e = end ? launch_pass<T, ADJOINT, false, true, false>(P, nullptr, source, out, nullptr, alpha, stream)
-                    : launch_pass<T, ADJOINT, false, true, true>(P, nullptr, source, nullptr, dst, alpha, stream);
-        source = dst;
+        const bool end = out && s == steps - 1;
+        const pass_io io{fields, source, end ? out : nullptr, source == a ? b : a};
+        if (!source) e = end ? launch_fields<T, ADJOINT, false>(P, io, alpha, stream) : launch_fields<T, ADJOINT, true>(P, io, alpha, stream);
+        else if (TWICE && s == 0) e = end ? launch_tiles<T, ADJOINT, TWICE, false>(P, io, alpha, stream) : launch_tiles<T, ADJOINT, TWICE, true>(P, io, alpha, stream);
+        else e = end ? launch_tiles<T, ADJOINT, false, false>(P, io, alpha, stream) : launch_tiles<T, ADJOINT, false, true>(P, io, alpha, stream);
+        fields = nullptr, source = io.packed;
     }
     return e;
 }

@@ -31,6 +31,13 @@ struct ghexb_program_s
     int32_t halo = 1;
     int64_t packed_elements = 0;
     std::vector<ghexb::program_domain> domains; // one per field
+    // device word: bit 0, a load of a pass did not arrive in time (its outputs are not written)
+    unsigned* status = nullptr;
+
+    ~ghexb_program_s()
+    {
+        if (status) cudaFree(status);
+    }
 };
 
 namespace ghexb

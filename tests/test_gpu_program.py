@@ -55,6 +55,7 @@ CASES = [
     ((24, 18, 20), (2, 2, 2), (True, False, True), 2, None),
     ((24, 20, 12), (4, 3, 3), (True, True, True), 1, None),
     ((300, 40, 9), (2, 2, 1), (True, True, True), 1, 2),
+    ((270, 150, 70), (2, 1, 1), (True, True, True), 1, 3),
 ]
 
 
@@ -84,6 +85,7 @@ def test_fused_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
         assert equal(*fields)
         assert equal(*ins)
         assert equal(*grads)
+    assert dx._program(halo).status() == 0
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
