@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+from array import array as _array
 import os
 import threading
 from typing import Any, Iterable, Sequence
@@ -31,6 +32,16 @@ class Architecture(enum.Enum):
 # --------------------------------------------------------------------------------------------
 _TYPESTR = {"<f4": _capi.F32, "<f8": _capi.F64, "<i4": _capi.I32, "<i8": _capi.I64,
             "|u1": _capi.U8, "<u2": _capi.U16}
+
+
+_codes: dict = {}
+
+
+def _torch_codes(torch) -> dict:
+    if not _codes:
+        _codes.update({torch.float32: _capi.F32, torch.float64: _capi.F64, torch.int32: _capi.I32,
+                       torch.int64: _capi.I64, torch.uint8: _capi.U8, torch.uint16: _capi.U16})
+    return _codes
 
 
 def _torch():
@@ -62,8 +73,7 @@ def array_info(field: Any) -> dict:
     if torch is not None and isinstance(field, torch.Tensor):
         if not field.is_cuda and field.device.type != "cpu":
             raise TypeError(f"unsupported tensor device {field.device}")
-        codes = {torch.float32: _capi.F32, torch.float64: _capi.F64, torch.int32: _capi.I32,
-                 torch.int64: _capi.I64, torch.uint8: _capi.U8, torch.uint16: _capi.U16}
+        codes = _torch_codes(torch)
         if field.dtype not in codes:
             raise TypeError(f"unsupported dtype {field.dtype}")
         es = field.element_size()
@@ -198,9 +208,22 @@ def stream_of(fields: Iterable[Any]):
     torch = _torch()
     for f in fields:
         if torch is not None and isinstance(f, torch.Tensor):
-            dev = f.device if f.is_cuda else None  # pinned host tensors: the current device's stream
-            return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+            # pinned host tensors: the current device's stream
+            return C.c_void_p(_raw_stream(f.get_device() if f.is_cuda else torch.cuda.current_device()))
     return C.c_void_p(0)
+
+
+def _raw_stream(device: int) -> int:
+    """The address of torch's current stream on a device (without a stream object, where torch has
+    the call for it)."""
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device) if raw is not None else torch.cuda.current_stream(device).cuda_stream
+
+
+def _stream_of_bound(bis: Sequence["BufferInfo"]):
+    """stream_of the arrays of buffer_infos."""
+    return stream_of(bi.field.array for bi in bis)
 
 
 # --------------------------------------------------------------------------------------------
@@ -245,14 +268,22 @@ def make_context(comm: Any = None, thread_safe: bool = False, device: int | None
 class BufferInfo:
     """A field bound to a pattern (buffer_info.hpp:33-71). Holds references, owns nothing."""
 
-    __slots__ = ("pattern", "field")
+    __slots__ = ("pattern", "field", "_value")
 
     def __init__(self, pattern: "PatternContainer", field: "FieldDescriptorBase"):
         self.pattern = pattern
         self.field = field
+        self._value = 0
 
     def handle(self) -> C.c_void_p:
         return self.field._bind(self.pattern)
+
+    def value(self) -> int:
+        """The handle as a number, looked up once: a field's binding to a pattern lasts as long as
+        the field, which this object keeps."""
+        if not self._value:
+            self._value = self.handle().value
+        return self._value
 
     def arrays(self) -> list:
         return [self.field.array]
@@ -378,6 +409,8 @@ def wrap_spec(pattern: PatternContainer, spec: dict, ptr: int) -> C.c_void_p:
 def _flatten(args: tuple) -> list[BufferInfo]:
     if len(args) == 1 and isinstance(args[0], (list, tuple)):
         args = tuple(args[0])
+    if set(map(type, args)) == {BufferInfo}:
+        return list(args)
     out = []
     for a in args:
         if isinstance(a, (list, tuple)):
@@ -402,7 +435,9 @@ class Handle:
         self._keep = keep
 
     def wait(self) -> None:
-        call("ghexb_handle_wait", self._h)
+        rc = _capi.handle_wait(self._h)
+        if rc:
+            _capi.check(rc)
         self._keep = []
 
     def is_ready(self) -> bool:
@@ -437,11 +472,12 @@ class CommunicationObject:
 
     def exchange(self, *buffer_infos) -> Handle:
         bis = _flatten(buffer_infos)
-        handles = (C.c_void_p * len(bis))(*[bi.handle() for bi in bis])
-        arrays = [a for bi in bis for a in bi.arrays()]
+        handles = _array("Q", [bi._value or bi.value() for bi in bis])
         h = C.c_void_p()
-        call("ghexb_co_exchange", self._h, handles, len(bis), stream_of(arrays), C.byref(h))
-        return Handle(self, h, [bis, arrays])
+        rc = _capi.co_exchange(self._h, handles.buffer_info()[0], len(bis), _stream_of_bound(bis), C.byref(h))
+        if rc:
+            _capi.check(rc)
+        return Handle(self, h, [bis])
 
     def __del__(self, _release=_capi.release):
         _release("ghexb_co_destroy", getattr(self, "_h", None))

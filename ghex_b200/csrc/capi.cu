@@ -10,6 +10,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <unordered_map>
 
 #include "exchange.hpp"
 #include "ipc.hpp"
@@ -55,26 +56,23 @@ void require(bool cond, const char* msg)
     if (!cond) throw ghexb::error(GHEXB_ERR_INVALID, msg);
 }
 
-std::vector<int64_t> signature(const ghexb_field* fields, int n)
+// What two fields must share to be exchanged by one plan: everything but the handle.
+bool same_field(const ghexb_field_s& a, const ghexb_field_s& b)
 {
-    std::vector<int64_t> s;
+    return a.pattern == b.pattern && a.domain_index == b.domain_index && a.dtype == b.dtype && a.data == b.data && a.ndim == b.ndim &&
+           a.offsets == b.offsets && a.extents == b.extents && a.byte_strides == b.byte_strides && a.layout == b.layout &&
+           a.num_components == b.num_components && a.is_vector == b.is_vector && a.levels == b.levels &&
+           a.levels_first == b.levels_first && a.index_stride == b.index_stride && a.level_stride == b.level_stride;
+}
+
+// A hash of the fields' memory, by which a communication object finds the plans to compare with.
+uint64_t fields_hash(const ghexb_field* fields, int n)
+{
+    uint64_t h = (uint64_t)n;
     for (int i = 0; i < n; ++i)
-    {
-        const auto& f = *fields[i];
-        s.push_back((int64_t)(intptr_t)f.pattern);
-        s.push_back(f.domain_index);
-        s.push_back(f.dtype);
-        s.push_back((int64_t)(intptr_t)f.data);
-        s.push_back(f.ndim);
-        for (int a = 0; a < 4; ++a) s.push_back(f.offsets[a]), s.push_back(f.extents[a]), s.push_back(f.byte_strides[a]), s.push_back(f.layout[a]);
-        s.push_back(f.num_components);
-        s.push_back(f.is_vector);
-        s.push_back(f.levels);
-        s.push_back(f.levels_first);
-        s.push_back(f.index_stride);
-        s.push_back(f.level_stride);
-    }
-    return s;
+        h = (h ^ (uint64_t)(uintptr_t)fields[i]->data ^ ((uint64_t)(uintptr_t)fields[i]->pattern << 17) ^ (uint64_t)fields[i]->domain_index) *
+            0x9E3779B97F4A7C15ull;
+    return h;
 }
 } // namespace
 
@@ -87,7 +85,7 @@ int set_last_error(int code, const std::string& msg) { return set_error(code, ms
 struct ghexb_co_s
 {
     ghexb_context_s* ctx = nullptr;
-    std::map<std::vector<int64_t>, std::unique_ptr<ghexb_plan_s>> plans;
+    std::unordered_multimap<uint64_t, std::unique_ptr<ghexb_plan_s>> plans; // by fields_hash
     bool in_place_receive = false;
     bool busy = false;
     cudaEvent_t done = nullptr;
@@ -640,15 +638,22 @@ int ghexb_co_exchange(ghexb_co co, const ghexb_field* fields, int n, void* strea
         require(n > 0, "an exchange needs at least one field");
         for (int i = 0; i < n; ++i) require(fields[i] != nullptr, "null field handle");
         if (co->busy) throw ghexb::error(GHEXB_ERR_BUSY, "earlier exchange operation was not finished");
-        auto key = signature(fields, n);
-        auto it = co->plans.find(key);
-        if (it == co->plans.end())
+        const uint64_t key = fields_hash(fields, n);
+        auto range = co->plans.equal_range(key);
+        auto it = std::find_if(range.first, range.second, [&](const auto& kv) {
+            const auto& f = kv.second->fields;
+            if ((int)f.size() != n) return false;
+            for (int i = 0; i < n; ++i)
+                if (!same_field(f[i], *fields[i])) return false;
+            return true;
+        });
+        if (it == range.second)
         {
             if (co->plans.size() >= 64) co->plans.clear();
             auto plan = std::make_unique<ghexb_plan_s>();
             plan->in_place_receive = co->in_place_receive;
             ghexb::build_plan(*plan, co->ctx, fields, n);
-            it = co->plans.emplace(std::move(key), std::move(plan)).first;
+            it = co->plans.emplace(key, std::move(plan));
         }
         if (!co->done) ghexb::check_cuda(cudaEventCreateWithFlags(&co->done, cudaEventDisableTiming), "cudaEventCreate");
         auto s = static_cast<cudaStream_t>(stream);
