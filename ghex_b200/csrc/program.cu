@@ -123,6 +123,27 @@ template <typename T> __device__ __forceinline__ cells<T> zero_if(bool z, const 
 
 constexpr int k_batch = 32; // domains per launch
 
+// Passes follow one another: a pass lets the next one be launched (programmatic stream serialisation)
+// when its blocks come to their last plane, so that the other's blocks start and set up their
+// barriers as its own leave; they wait for the whole of it before they touch any memory but their
+// arguments. 256 x 256 x 128 float32, 10 steps forward and back: 347 -> 336 us; 48 x 50 x 40: 102.7
+// -> 90.5. Let go at a block's start instead, the next pass's blocks settle in whatever slots are
+// free and leave some SMs with more of them than others: 330 and 101.7 us, and 64 x 200 x 60 157 us
+// where it had been 148 (at the last plane: 145).
+__device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void lead() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... Params, typename... Args>
+cudaError_t launch_following(void (*kernel)(Params...), unsigned blocks, unsigned threads, size_t shared, cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(blocks), config.blockDim = dim3(threads), config.dynamicSmemBytes = shared, config.stream = stream;
+    config.attrs = &attribute, config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
+
 // One domain of a launch; cell (0, 0, 0) is the first interior cell, strides count elements.
 struct pass_domain
 {
@@ -156,7 +177,10 @@ constexpr int k_threads = 128;
 constexpr int k_rows = 2;
 constexpr int k_stages = 3;
 constexpr int k_resident = 5; // blocks per SM
-constexpr int k_min_slab = 4; // planes
+// Planes of a slab at least: small domains take as many slabs as the chip holds blocks, so that a
+// block's loads are all under way at once (48 x 50 x 40 in 8 domains, 8 steps forward and back: 4
+// planes at least 90.5 us, 2 71.9, 1 64.2; 64 x 200 x 60, 10 steps: 144.9, 118.1, 118.0).
+constexpr int k_min_slab = 1;
 constexpr int k_halo_cells = 8; // halo cells a thread writes
 
 // a plane in the ring of a block: rows -1 .. R of 16 bytes per thread, then the cells beside the R rows
@@ -320,6 +344,7 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
     while (di + 1 < args.n && b >= args.d[di + 1].block0) ++di;
     const pass_domain& d = args.d[di];
     b -= d.block0;
+    follow();
     if (b >= d.marches)
     {
         if constexpr (!OUT_PACKED) write_halo<T, ADJOINT, false, k_threads>(d, alpha, b - d.marches);
@@ -427,6 +452,7 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
 #pragma unroll 1
     for (int k = k0; k < k1; ++k)
     {
+        if (k + 1 == k1) lead();
         issue(k + k_stages - 1, free_at);
         copy_wait<k_stages - 2>(); // plane k + 1 has landed
         const uint32_t up = here + ring<T>::stage == ring<T>::bytes ? 0 : here + ring<T>::stage;
@@ -520,6 +546,7 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
     b -= d.block0;
     if (b >= d.marches)
     {
+        follow();
         if constexpr (!OUT_PACKED) write_halo<T, ADJOINT, TWICE, k_tile_threads + 32>(d, alpha, b - d.marches);
         return;
     }
@@ -545,6 +572,7 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
         mbar_init_fence();
     }
     __syncthreads();
+    follow();
     // planes k0 - 1 .. k1 of the slab, numbered from 0
     const int planes = k1 - k0 + 2;
     const bool row_lo = y0 == 0 && face(2), row_hi = y0 + h >= ny && face(3);
@@ -647,6 +675,7 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
     for (int k = k0; k < k1; ++k)
     {
         const int q = k - k0 + 1;
+        if (k + 1 == k1) lead();
         issue_sides(q - 1 + S, st == 0 ? S - 1 : st - 1); // (a thread's own, read one plane ago)
         wait(up, up_parity);
         copy_wait<S - 1>(); // the sides of plane q
@@ -834,8 +863,7 @@ cudaError_t launch_fields(const ghexb_program_s& P, const pass_io& io, double al
         const auto kernel = pass_kernel<T, ADJOINT, OUT_PACKED>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring<T>::bytes);
         if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)blocks, k_threads, ring<T>::bytes, stream>>>(args, (T)alpha);
-        e = cudaGetLastError();
+        e = launch_following(kernel, (unsigned)blocks, k_threads, ring<T>::bytes, stream, args, (T)alpha);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -921,8 +949,7 @@ cudaError_t launch_tiles_r(const ghexb_program_s& P, const pass_io& io, double a
         const auto kernel = tile_kernel<T, ADJOINT, TWICE, OUT_PACKED, R>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)blocks, k_tile_threads + 32, bytes, stream>>>(args, (T)alpha);
-        e = cudaGetLastError();
+        e = launch_following(kernel, (unsigned)blocks, k_tile_threads + 32, bytes, stream, args, (T)alpha);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1105,6 +1132,7 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_kernel(const __grid_const
     while (di + 1 < args.n && b >= args.d[di + 1].block0) ++di;
     const auto& d = args.d[di];
     b -= d.block0;
+    follow();
     const uint64_t all = (uint64_t)d.chunks * d.ny * d.nz;
     const T* __restrict__ p = static_cast<const T*>(d.p);
     cells<T> c[k_sum_chunks];
@@ -1146,6 +1174,7 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_kernel(const __grid_const
 
 template <typename T> __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* __restrict__ partials, uint32_t n, T* out)
 {
+    follow();
     double s = 0;
     for (uint32_t i = threadIdx.x; i < n; i += 1024) s = __dadd_rn(s, partials[i]);
     s = block_sum(s);
@@ -1175,6 +1204,7 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_grad_kernel(const __grid_
     const auto& d = args.d[di];
     b -= d.block0;
     const int h = args.halo;
+    follow();
     const uint64_t all = (uint64_t)d.ex * d.ey * d.ez;
     const T scale = __ldg(g);
     const T* __restrict__ p = static_cast<const T*>(d.p);
@@ -1225,15 +1255,11 @@ cudaError_t launch_sumsq_t(const interior* d, int n, bool packed, double* partia
             blocks += sum_blocks(cells<T>::V, s.n);
         }
         if (done + blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-        if (packed) sumsq_kernel<T, true><<<(unsigned)blocks, k_sum_threads, 0, stream>>>(args, partials + done);
-        else
-            sumsq_kernel<T, false><<<(unsigned)blocks, k_sum_threads, 0, stream>>>(args, partials + done);
+        const cudaError_t e = launch_following(packed ? sumsq_kernel<T, true> : sumsq_kernel<T, false>, (unsigned)blocks, k_sum_threads, 0, stream, args, partials + done);
         done += blocks;
-        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    sum_partials_kernel<T><<<1, 1024, 0, stream>>>(partials, (uint32_t)done, static_cast<T*>(out));
-    return cudaGetLastError();
+    return launch_following(sum_partials_kernel<T>, 1, 1024, 0, stream, (const double*)partials, (uint32_t)done, static_cast<T*>(out));
 }
 
 template <typename T>
@@ -1255,8 +1281,7 @@ cudaError_t launch_grad_t(const interior* d, void* const* out, int n, int halo, 
             blocks += ((uint64_t)s.n[0] * s.n[1] * s.n[2] + per - 1) / per;
         }
         if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-        sumsq_grad_kernel<T><<<(unsigned)blocks, k_sum_threads, 0, stream>>>(args, static_cast<const T*>(g));
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_following(sumsq_grad_kernel<T>, (unsigned)blocks, k_sum_threads, 0, stream, args, static_cast<const T*>(g));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
