@@ -1000,6 +1000,15 @@ double run_cost(int64_t count, int unit, int64_t row)
     return (double)count * unit * (w + 32.0) / w;
 }
 
+// A forward tile's rows run along its first axis where source and destination are both
+// contiguous along it (pairs: segments of n0 elements); otherwise every element is a row.
+double tile_cost(const xtile& t)
+{
+    auto unit_stride = [](int32_t v) { return v == 1 || v == -1; };
+    const bool contiguous = t.kind == 2 || (t.kind == 0 ? unit_stride(t.s0) && unit_stride(t.d0) : t.s1 == 1 && t.d1 == 1);
+    return run_cost(t.count, t.unit, contiguous ? t.n0 : 1);
+}
+
 // Rows of a forward box or pair tile that are shorter than a 128-byte line; 0 for other tiles.
 double short_rows(const xtile& t)
 {
@@ -1787,7 +1796,7 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
             if ((int)plan.lists[i].field == lg) f.insert(f.end(), ltiles[i].begin(), ltiles[i].end());
         plan.xp_field[lg] = append_range(plan.xp, f);
     }
-    // batched: one range, field by field; staged boxes are the staged kernel's, and
+    // batched: one range, ordered below; staged boxes are the staged kernel's, and
     // a pair moves as a pair only when neither of its boxes is staged
     {
         auto paired = [&](int i) {
@@ -1879,29 +1888,41 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
                 plan.bt_col0.push_back(c0);
             }
         }
-        // Field by field, each in the order of its descriptors (by receiving domain). The rows that the
-        // faces of a domain read and those that they write share 128-byte lines, as do a row's end and
-        // the next row's start, so lines that stay in the L2 between two tiles are fetched once and
-        // written back whole; and short and long rows run side by side, which the most expensive rows
-        // first kept apart: 3 x 3 x 3 uneven domains of 800 x 600 x 192, five fields, 180 -> 162 us. A
-        // field whose short rows hold more lines than the L2 goes in bins of the same fraction of
-        // every descriptor (the same rows and levels of every face): cubed sphere of edge 384, 90
-        // levels, 178 -> 163 us (DRAM reads 369 -> 323 MB, the distinct lines 313 MB); four bins where
-        // the lines fit cost the regular case 174 us.
-        std::map<uint32_t, double> lines; // bytes of the lines of a field's short rows
-        for (size_t i = 0; i < all.size(); ++i)
-            if (const double rows = short_rows(all[i])) lines[all_at[i].first] += rows * 128.0;
-        std::vector<std::array<uint32_t, 3>> order(all.size()); // field, bin, tile
-        for (size_t i = 0; i < all.size(); ++i)
+        std::vector<double> lines(plan.n_logical, 0.0); // bytes of the lines of a field's short rows
+        double all_lines = 0;
+        for (size_t i = 0; i < all.size(); ++i) lines[all_at[i].first] += short_rows(all[i]) * 128.0;
+        for (double l : lines) all_lines += l;
+        if (all_lines <= k_order_bytes)
         {
-            const auto it = lines.find(all_at[i].first);
-            const double bins = it == lines.end() ? 1.0 : 1.0 + std::floor(it->second / k_order_bytes);
-            order[i] = {all_at[i].first, (uint32_t)(all_at[i].second * bins), (uint32_t)i};
+            // the most DRAM bytes per element (short rows) first: the first wave of CTAs starts on the most
+            // expensive tiles (2 x 3 x 2 domains of 271 x 194 x 78, five fields: 11.1 us, by field 12.2)
+            auto per_elem = [](const xtile& t) { return tile_cost(t) / std::max<uint32_t>(1u, t.count); };
+            std::stable_sort(all.begin(), all.end(), [&](const xtile& x, const xtile& y) { return per_elem(x) > per_elem(y); });
         }
-        std::sort(order.begin(), order.end());
-        std::vector<xtile> sorted(all.size());
-        for (size_t i = 0; i < all.size(); ++i) sorted[i] = all[order[i][2]];
-        all.swap(sorted);
+        else
+        {
+            // Lines that the L2 does not hold: field by field, each in the order of its descriptors (by
+            // receiving domain). The rows that the faces of a domain read and those that they write share
+            // 128-byte lines, as do a row's end and the next row's start, so lines that stay in the L2
+            // between two tiles are fetched once and written back whole; and short and long rows run side
+            // by side: 3 x 3 x 3 uneven domains of 800 x 600 x 192, five fields, 180 -> 162 us. A field
+            // whose short rows alone hold more lines than the L2 goes in bins of the same fraction of
+            // every descriptor (the same rows and levels of every face): cubed sphere of edge 384, 90
+            // levels, 178 -> 163 us (DRAM reads 369 -> 323 MB, the distinct lines 313 MB); four bins where
+            // a field's lines fit cost the regular case 174 us. (400 x 300 x 96, whose lines of 79 MB fit,
+            // takes 62 us either way.)
+            std::vector<std::pair<uint64_t, uint32_t>> order(all.size()); // field and bin, tile
+            for (size_t i = 0; i < all.size(); ++i)
+            {
+                const uint32_t field = all_at[i].first;
+                const uint32_t bin = (uint32_t)(all_at[i].second * (1.0 + std::floor(lines[field] / k_order_bytes)));
+                order[i] = {(uint64_t)field << 32 | bin, (uint32_t)i};
+            }
+            std::sort(order.begin(), order.end());
+            std::vector<xtile> sorted(all.size());
+            for (size_t i = 0; i < all.size(); ++i) sorted[i] = all[order[i].second];
+            all.swap(sorted);
+        }
         plan.xf.clear();
         append_range(plan.xf, all);
     }

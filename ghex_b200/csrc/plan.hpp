@@ -45,8 +45,8 @@ struct ghexb_plan_s
     std::vector<int64_t> adj_src_off, adj_dst_off;
     int n_logical = 0;
 
-    // Forward work (exchange.cu), one CTA per tile: xf is the batched form's table (field
-    // by field), xp the per-field form's (grouped by logical field) and xb
+    // Forward work (exchange.cu), one CTA per tile: xf is the batched form's table (the most
+    // DRAM bytes per element first or, in large exchanges, field by field), xp the per-field form's (grouped by logical field) and xb
     // the per-box form's (grouped by descriptor).
     std::vector<ghexb::xtile> xf, xp, xb;
     // Index blocks of the list tiles, one per tile of xf, xp and xb (exchange.hpp
