@@ -111,7 +111,8 @@ struct alignas(16) list_desc
 // 112-byte record and nothing else before its data loads.
 //  * box:  element e -> i0 = e mod n0, r = e / n0, i1 = r mod n1, i2 = r / n1;
 //          dst[i0*d0 + i1*d1 + i2*d2] = src[i0*s0 + i1*s1 + i2*s2]  (sign bit flipped if neg)
-//  * list: element e -> k = e / n0 (column), l = e mod n0 (level);
+//  * list: element e -> k = e / n0 (column), l = e mod n0 (level) or, of tiles of n1 > 1 columns,
+//          l = (e - e0) / n1, k = e0 / n0 + (e - e0) mod n1;
 //          dst[didx[k]*d0 + l*d1] = src[sidx[k]*s0 + l*s1]
 //  * pair: two boxes A and B of short rows in one destination field whose rows interleave in
 //          memory: row r of A ends where row r + 1 of B begins (the high-x halo of a row and the
@@ -154,7 +155,8 @@ constexpr int k_xtile_words = 7;
 // which is the explicit transpose in receive order, with no two threads touching one element.
 // Unstructured columns take the same form: a group of owner columns with the same number of
 // images; the column table holds, per owner, the address of its column and of each image's
-// column (nimg + 1 addresses), and element e of the group is level e mod n0 of owner e / n0.
+// column (nimg + 1 addresses), and element e of the group is level e mod n0 of owner e / n0
+// (of tiles of n1 > 1 whole columns: of owner e0 / n0 + (e - e0) mod n1, level (e - e0) / n1).
 constexpr int k_max_images = 8;
 
 struct gimage

@@ -121,7 +121,9 @@ __device__ __forceinline__ void box_elements(const xtile& t)
 
 // blk: the tile's index block in shared memory (the indices of columns t.u0, t.u0 + 1, ...), or
 // nullptr when the tile reads its indices from the lists
-template<int K, typename T>
+// COLUMNS: neighbouring threads take neighbouring columns (a code of its own: a branch per element
+// cost the other form 8 %)
+template<int K, typename T, bool COLUMNS = false>
 __device__ __forceinline__ void list_elements(const xtile& t, const int32_t* blk)
 {
     const T* __restrict__ src = reinterpret_cast<const T*>(t.src);
@@ -135,9 +137,19 @@ __device__ __forceinline__ void list_elements(const xtile& t, const int32_t* blk
         doff[k] = 0;
         if (e < t.count)
         {
-            const uint32_t g = t.e0 + e;
-            const uint32_t col = fdiv(g, t.m0, t.l0);
-            const int32_t lev = (int32_t)(g - col * t.n0);
+            uint32_t col;
+            int32_t lev;
+            if constexpr (COLUMNS)
+            {
+                const uint32_t l = fdiv(e, t.m1, t.l1);
+                col = (uint32_t)t.u0 + (e - l * t.n1), lev = (int32_t)l;
+            }
+            else
+            {
+                const uint32_t g = t.e0 + e;
+                col = fdiv(g, t.m0, t.l0);
+                lev = (int32_t)(g - col * t.n0);
+            }
             if (blk)
             {
                 const uint32_t c = col - (uint32_t)t.u0;
@@ -234,10 +246,13 @@ __global__ void __launch_bounds__(k_max_block, K >= 16 ? 1 : 2) exchange_kernel(
         GHEXB_CASE(k_box2, (box_elements<K, uint16_t, false>))
         GHEXB_CASE(k_box1, (box_elements<K, uint8_t, false>))
         case k_list16: list_elements<forward_per_thread(K, 16), uint4>(t, blk); break;
-        case k_list8: list_elements<K, unsigned long long>(t, blk); break;
-        case k_list4: list_elements<K, uint32_t>(t, blk); break;
-        case k_list2: list_elements<K, uint16_t>(t, blk); break;
-        case k_list1: list_elements<K, uint8_t>(t, blk); break;
+#define GHEXB_LIST(C, T)                                                                                               \
+    case C: t.n1 > 1 ? list_elements<K, T, true>(t, blk) : list_elements<K, T>(t, blk); break;
+        GHEXB_LIST(k_list8, unsigned long long)
+        GHEXB_LIST(k_list4, uint32_t)
+        GHEXB_LIST(k_list2, uint16_t)
+        GHEXB_LIST(k_list1, uint8_t)
+#undef GHEXB_LIST
         GHEXB_CASE(k_pair8, (pair_elements<K, unsigned long long>))
         GHEXB_CASE(k_pair4, (pair_elements<K, uint32_t>))
 #undef GHEXB_CASE
@@ -299,7 +314,7 @@ __device__ __forceinline__ void gather_elements(const gtile& t)
 
 // Unstructured owner columns: element e is level e mod n0 of owner e / n0 of the group; the
 // owner's and its images' column addresses come from the column table.
-template<int K, int NI, typename F>
+template<int K, int NI, typename F, bool COLUMNS>
 __device__ __forceinline__ void list_gather_elements(const gtile& t, const uint64_t* __restrict__ cols,
     const uint64_t* blk)
 {
@@ -307,12 +322,22 @@ __device__ __forceinline__ void list_gather_elements(const gtile& t, const uint6
     F acc[K];
     // the tile's columns from its block in shared memory, else from the column table; a column's
     // address is looked up again for the stores rather than held in registers across the loads
-    const uint32_t j0 = blk ? fdiv(t.e0, t.m0, t.l0) : 0u;
+    const uint32_t first = fdiv(t.e0, t.m0, t.l0), j0 = blk ? first : 0u;
     const uint64_t* base = blk ? blk - (size_t)j0 * (NI + 1) : cols + t.col0;
     auto column = [&](uint32_t e, int i) {
-        const uint32_t g = t.e0 + e;
-        const uint32_t j = fdiv(g, t.m0, t.l0);
-        const int32_t lev = (int32_t)(g - j * t.n0);
+        uint32_t j;
+        int32_t lev;
+        if constexpr (COLUMNS)
+        {
+            const uint32_t l = fdiv(e, t.m1, t.l1);
+            j = first + (e - l * t.n1), lev = (int32_t)l;
+        }
+        else
+        {
+            const uint32_t g = t.e0 + e;
+            j = fdiv(g, t.m0, t.l0);
+            lev = (int32_t)(g - j * t.n0);
+        }
         const uint64_t* p = base + (size_t)j * (NI + 1) + i;
         return reinterpret_cast<F*>(blk ? *p : __ldg(p)) + lev * (i == 0 ? t.o0 : t.img[0].t0);
     };
@@ -382,11 +407,17 @@ __global__ void __launch_bounds__(k_gather_block, 4) list_gather_kernel(const gt
             __ldg(reinterpret_cast<const uint4*>(blocks + (size_t)blockIdx.x * k_gblock_entries) + (threadIdx.x - 16));
     load_record<16>(t, tiles);
     const uint64_t* blk = blocks && t.pad[0] ? blk_s : nullptr;
-    switch (t.cls)
+    switch (t.cls + (t.n1 > 1 ? k_gather_classes : 0))
     {
 #define GHEXB_CASE(NI)                                                                                                 \
-    case list_gather_class(8, NI): list_gather_elements<gather_per_thread(NI), NI, double>(t, cols, blk); break;     \
-    case list_gather_class(4, NI): list_gather_elements<gather_per_thread(NI), NI, float>(t, cols, blk); break;
+    case list_gather_class(8, NI): list_gather_elements<gather_per_thread(NI), NI, double, false>(t, cols, blk); break;  \
+    case list_gather_class(4, NI): list_gather_elements<gather_per_thread(NI), NI, float, false>(t, cols, blk); break;   \
+    case k_gather_classes + list_gather_class(8, NI):                                                                   \
+        list_gather_elements<gather_per_thread(NI), NI, double, true>(t, cols, blk);                                    \
+        break;                                                                                                          \
+    case k_gather_classes + list_gather_class(4, NI):                                                                   \
+        list_gather_elements<gather_per_thread(NI), NI, float, true>(t, cols, blk);                                     \
+        break;
         GHEXB_CASE(1)
         GHEXB_CASE(2)
         GHEXB_CASE(3)

@@ -1708,27 +1708,46 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
     };
     auto list_tiles = [&](int i, std::vector<xtile>& out) {
         const auto& l = plan.lists[i];
-        const fast_div f0 = fast_div::make((uint32_t)l.levels);
-        const uint32_t n = (uint32_t)((int64_t)l.count * l.levels);
-        uint32_t c = row_cap((int)l.unit, l.levels);
-        // whole columns, at most k_block_columns of them, when a tile holds at least one: the
-        // tile's index block (below) then covers its columns
-        if ((uint32_t)l.levels <= c) c = std::min<uint32_t>(c / l.levels, k_block_columns) * (uint32_t)l.levels;
-        for (uint32_t e0 = 0; e0 < n; e0 += c)
-        {
+        auto tile = [&](uint32_t levels, uint32_t level0, uint32_t e0, uint32_t count) {
+            const fast_div f0 = fast_div::make(levels);
             xtile t{};
-            t.src = l.src, t.dst = l.dst;
+            t.src = l.src + (int64_t)level0 * l.s_ls * l.unit, t.dst = l.dst + (int64_t)level0 * l.d_ls * l.unit;
             t.sidx = idx ? idx + plan.list_idx_off[i] : nullptr;
             t.didx = idx ? idx + plan.list_idx_off[i] + l.count : nullptr;
-            t.e0 = e0, t.count = std::min(c, n - e0);
+            t.e0 = e0, t.count = count;
             t.s0 = l.s_is, t.s1 = l.s_ls, t.d0 = l.d_is, t.d1 = l.d_ls;
             t.n0 = f0.d, t.m0 = f0.m, t.l0 = (uint8_t)f0.l;
             t.n1 = 1, t.m1 = 1, t.l1 = 0;
             t.unit = (uint8_t)l.unit;
             t.kind = 1;
-            t.u0 = (int32_t)(e0 / (uint32_t)l.levels); // first column of the tile
-            out.push_back(t);
+            t.u0 = (int32_t)(e0 / levels); // first column of the tile
+            return t;
+        };
+        // Columns whose levels lie further apart than their neighbours: a tile is up to
+        // k_block_columns columns by some of the levels, and neighbouring threads take neighbouring
+        // columns (n1 of them), whose indices mostly follow one another. 16 domains of 512 x 768
+        // columns, 30 levels, float64: 8.15 -> 6.18 us; 800 x 900, 90 levels, float64 and
+        // float32: 36.9 -> 26.7 us.
+        if (l.levels > 1 && l.s_ls > l.s_is && l.d_ls > l.d_is)
+        {
+            const uint32_t nl = std::min<uint32_t>(std::max<uint32_t>(1u, cap((int)l.unit) / k_block_columns), (uint32_t)l.levels);
+            for (uint32_t level0 = 0; level0 < (uint32_t)l.levels; level0 += nl)
+                for (uint32_t c0 = 0; c0 < (uint32_t)l.count; c0 += k_block_columns)
+                {
+                    const uint32_t levels = std::min(nl, (uint32_t)l.levels - level0), columns = std::min<uint32_t>(k_block_columns, l.count - c0);
+                    xtile t = tile(levels, level0, c0 * levels, columns * levels);
+                    const fast_div f1 = fast_div::make(columns);
+                    t.n1 = f1.d, t.m1 = f1.m, t.l1 = (uint8_t)f1.l;
+                    out.push_back(t);
+                }
+            return;
         }
+        const uint32_t n = (uint32_t)((int64_t)l.count * l.levels);
+        uint32_t c = row_cap((int)l.unit, l.levels);
+        // whole columns, at most k_block_columns of them, when a tile holds at least one: the
+        // tile's index block (below) then covers its columns
+        if ((uint32_t)l.levels <= c) c = std::min<uint32_t>(c / l.levels, k_block_columns) * (uint32_t)l.levels;
+        for (uint32_t e0 = 0; e0 < n; e0 += c) out.push_back(tile((uint32_t)l.levels, 0, e0, std::min(c, n - e0)));
     };
     auto pair_tiles = [&](int p, std::vector<xtile>& out) {
         const auto& A = plan.boxes[plan.pairs[p].first];
@@ -2032,8 +2051,14 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
             }
             // the other owners of the group: element tiles of list_gather_kernel
             const uint32_t col0 = group0 + (uint32_t)(nb * per);
-            const uint32_t gc = (uint32_t)(gather_per_thread(o0.nimg) * k_gather_block);
+            uint32_t gc = (uint32_t)(gather_per_thread(o0.nimg) * k_gather_block);
             const uint32_t n = (uint32_t)((int64_t)(b - a - nb) * o0.levels);
+            // levels further apart than columns (as the forward's list tiles): whole columns, as many
+            // as the block of column addresses holds, and neighbouring threads take neighbouring columns
+            // (16.1 -> 10.9 and 79.9 -> 56.8 us on the two sizes there)
+            const auto& of = plan.fields[o0.slot];
+            const bool by_column = o0.levels > 1 && of.level_stride > of.index_stride && (uint32_t)o0.levels <= gc;
+            if (by_column) gc = std::min(gc / (uint32_t)o0.levels, std::min<uint32_t>(32u, (uint32_t)k_gblock_entries / per)) * (uint32_t)o0.levels;
             const fast_div f0 = fast_div::make((uint32_t)o0.levels);
             for (uint32_t e0 = 0; e0 < n; e0 += gc)
             {
@@ -2047,6 +2072,11 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
                 t.nimg = (uint8_t)o0.nimg;
                 t.kind = 1;
                 t.col0 = col0;
+                if (by_column)
+                {
+                    const fast_div f1 = fast_div::make(t.count / t.n0);
+                    t.n1 = f1.d, t.m1 = f1.m, t.l1 = (uint8_t)f1.l;
+                }
                 t.cls = (uint8_t)class_of_g(t);
                 plan.gt.push_back(t);
             }

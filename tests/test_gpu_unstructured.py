@@ -250,3 +250,26 @@ def test_receive_domain_ids_generator(levels):
         plan.adjoint()
         torch.cuda.synchronize()
         assert sum(bits_equal(t.cpu().numpy(), e) for t, e in zip(tens, adj)) == 0
+
+
+@pytest.mark.parametrize("levels", [2, 7, 33, 256, 300])
+@pytest.mark.parametrize("ni,nj,parts", [(6, 9, 4), (40, 52, 4), (131, 70, 8)])
+def test_level_major_tiles_bitexact(cuda, ni, nj, parts, levels):
+    """Fields stored level by level: tiles of 32 columns by some of the levels (one column, ends of
+    both, more levels than a descriptor holds), forward and adjoint, against the oracle. (The adjoint
+    adds halos, so its fields have gradients there in place of NaN.)"""
+    w = W.config2(ni=ni, nj=nj, parts=parts, levels=levels)
+    odoms = [OU.Domain(*d) for d in w.domains]
+    recv, send, _ = OU.make_pattern(odoms)
+    for form in ("batched", "per_box", "adjoint"):
+        fields = [[w.domain_array(d, t, s, False) for d in w.domains] for s, t in enumerate((np.float64, np.float32))]
+        if form == "adjoint":
+            rng = np.random.default_rng(9)
+            fields = [[np.asfortranarray(rng.standard_normal(x.shape).astype(x.dtype)) for x in f] for f in fields]
+        if form != "adjoint":
+            fields.append([(x * 100).astype(np.uint8, order="K") for x in fields[0]])
+        got = run_device(U.make_context(), w.domains, [[x.copy(order="K") for x in f] for f in fields], form)
+        for f, g in zip(fields, got):
+            assert f[0].strides[1] > f[0].strides[0]
+            (OU.adjoint if form == "adjoint" else OU.exchange)(recv, send, f)
+            assert sum(bits_equal(a, e) for a, e in zip(g, f)) == 0
