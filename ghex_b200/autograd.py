@@ -124,8 +124,7 @@ class DifferentiableExchange:
         ghexb_program_create refuses (then the two run one after the other)."""
         if halo not in self._programs:
             program = None
-            dense = all(torch.empty_like(t).stride() == t.stride() for t in
-                        (torch.empty_strided(sh, st, dtype=dt, device="meta") for sh, st, dt, _ in self._tensor_layout))
+            dense = all(_dense(shape, stride) for shape, stride, *_ in self._tensor_layout)
             if dense and len({dev for *_, dev in self._tensor_layout}) == 1 and self._tensor_layout[0][3].type == "cuda":
                 try:
                     program = _Program(self._bis, halo)
@@ -219,6 +218,16 @@ class Stencil7(torch.autograd.Function):
 def stencil7(xs: Sequence[torch.Tensor], alpha: float = 0.1, halo: int = 1):
     out = Stencil7.apply(alpha, halo, *xs)
     return out if isinstance(out, tuple) else (out,)
+
+
+def _dense(shape, stride) -> bool:
+    """Whether torch.empty_like keeps the strides: the elements fill their memory without gaps or overlaps."""
+    n = 1
+    for st, size in sorted((st, size) for size, st in zip(shape, stride) if size != 1):
+        if st != n:
+            return False
+        n *= size
+    return True
 
 
 class _Program:
