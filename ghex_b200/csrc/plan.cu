@@ -1823,11 +1823,12 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
             return !staged(pr.first) && !staged(pr.second);
         };
         std::vector<xtile> all;
-        std::vector<std::pair<uint32_t, double>> all_at; // per tile: its field, the fraction of its descriptor before it
+        // per tile: its field, the fraction of its descriptor's tiles before it (not e0, which starts
+        // again for every group of levels of a level-major list)
+        std::vector<std::pair<uint32_t, double>> all_at;
         all.reserve(plan.xb.size()), all_at.reserve(plan.xb.size());
         auto add = [&](const std::vector<xtile>& tiles, uint32_t field) {
-            const double n = tiles.empty() ? 1.0 : (double)tiles.back().e0 + tiles.back().count;
-            for (const auto& t : tiles) all.push_back(t), all_at.push_back({field, t.e0 / n});
+            for (size_t k = 0; k < tiles.size(); ++k) all.push_back(tiles[k]), all_at.push_back({field, (double)k / tiles.size()});
         };
         for (size_t i = 0; i < plan.boxes.size(); ++i)
             if (!staged((int)i) && !paired((int)i)) add(btiles[i], plan.boxes[i].field);
