@@ -606,11 +606,12 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
         }
         return;
     }
-    // the cells beyond x- and x+ beside this thread's rows
+    // the cells beyond x- and x+ beside this thread's rows (only a thread with a column of its own
+    // writes them: the others stand on the last column, and their warps may be planes ahead of it)
     const bool side_lo = first && face(0), side_hi = last && face(1);
     const uint32_t side = g.side0 + (uint32_t)(s * R) * (uint32_t)sizeof(T), side_other = side + (uint32_t)h * (uint32_t)sizeof(T);
     const auto issue_sides = [&](int q, int st) {
-        if ((side_lo || side_hi) && q > 0 && q + 1 < planes)
+        if (live && (side_lo || side_hi) && q > 0 && q + 1 < planes)
         {
             const uint32_t at = smem_u32(shared + (uint32_t)st * g.stage);
             const int k = k0 - 1 + q;

@@ -88,6 +88,31 @@ def test_fused_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
     assert dx._program(halo).status() == 0
 
 
+def check_fields_and_gradients(cuda, dx, x0, steps, halo, repeats):
+    leaves = [x.clone().requires_grad_(True) for x in x0]
+    _, ys = separately(dx, [x.clone() for x in leaves], steps, halo)
+    weights = [torch.linspace(-1, 1, y.numel(), dtype=y.dtype, device=cuda).reshape(y.shape) for y in ys]
+    grads = torch.autograd.grad(sum((y * v).sum() for y, v in zip(ys, weights)), leaves)
+    for _ in range(repeats):
+        zs = AG.diffusion_program(dx, [x.clone() for x in leaves], steps, ALPHA, halo)
+        assert equal(zs, ys)
+        assert equal(torch.autograd.grad(sum((z * v).sum() for z, v in zip(zs, weights)), leaves), grads)
+    assert dx._program(halo).status() == 0
+
+
+@pytest.mark.parametrize("shape,parts,dtype", [
+    ((48, 48, 400), (3, 3, 2), np.float64),    # 32 columns of a tile, 7 planes of a slab
+    ((96, 96, 192), (3, 3, 3), np.float64),    # 64, 7
+    ((64, 64, 400), (2, 2, 2), np.float64),    # 64, 6
+    ((193, 79, 180), (3, 3, 2), np.float32),   # 56, 6
+])
+def test_tiles_of_few_columns(cuda, shape, parts, dtype):
+    """Tiles that leave whole warps without a column, in slabs of more planes than are in flight: the
+    cells beside a row are written by its own thread only."""
+    dx, x0 = make(cuda, shape, parts, (True, True, True), 1, dtype, None)
+    check_fields_and_gradients(cuda, dx, x0, 4, 1, 4)
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("shape,parts,periodic,halo,seed", CASES[:1] + CASES[3:6])
 def test_graphed_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
