@@ -877,11 +877,12 @@ void shape_tile(tile_domain& t, uint32_t chunks, uint32_t strips, int V, int row
     double least = 0;
     t.cw = 0;
     const uint32_t widest = std::min<uint32_t>(k_tile_threads, 256u / V - 2u); // a load box is at most 256 elements wide
+    const uint32_t tallest = (256u - 2u) / (uint32_t)rows; // and at most 256 rows high, the ones around the tile among them
     const uint32_t few = (chunks + widest - 1) / widest;
     for (uint32_t nt = few; nt <= std::min(chunks, few + 16); ++nt)
     {
         const uint32_t cw = (chunks + nt - 1) / nt;
-        const uint32_t hs = std::min(std::min((uint32_t)k_tile_threads / cw, strips), 64u);
+        const uint32_t hs = std::min(std::min((uint32_t)k_tile_threads / cw, strips), tallest);
         const double blocks = (double)((chunks + cw - 1) / cw) * ((strips + hs - 1) / hs);
         const double cost = blocks * (1.0 + (double)(cw + 2) * (hs * rows + 2) / (k_tile_threads * rows));
         if (t.cw == 0 || cost < least) t.cw = cw, t.strips = hs, least = cost;

@@ -113,6 +113,23 @@ def test_tiles_of_few_columns(cuda, shape, parts, dtype):
     check_fields_and_gradients(cuda, dx, x0, 4, 1, 4)
 
 
+@pytest.mark.parametrize("shape,parts,dtype", [
+    ((4, 300, 8), (2, 1, 1), np.float64),      # a chunk wide, 75 strips of rows
+    ((8, 300, 8), (2, 1, 1), np.float32),
+    ((4, 256, 8), (1, 1, 2), np.float64),      # two chunks wide, 64 strips
+    ((16, 512, 6), (2, 2, 1), np.float32),
+    ((4, 252, 8), (2, 1, 1), np.float64),      # 63 strips
+])
+def test_narrow_long_domains(cuda, shape, parts, dtype):
+    """Domains of a chunk or two along x and of more rows than a load box is high."""
+    dx, x0 = make(cuda, shape, parts, (True, True, True), 1, dtype, None)
+    assert dx._program(1) is not None
+    check_fields_and_gradients(cuda, dx, x0, 3, 1, 1)
+    graphed = AG.GraphedDiffusion(dx, x0, 3, ALPHA)
+    _, ys = separately(dx, [x.clone() for x in x0], 3, 1)
+    assert equal([graphed.run(x0)[0]], [AG.interior_loss(ys)])
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("shape,parts,periodic,halo,seed", CASES[:1] + CASES[3:6])
 def test_graphed_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
