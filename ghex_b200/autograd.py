@@ -383,7 +383,8 @@ def interior_loss(xs: Sequence[torch.Tensor], halo: int = 1) -> torch.Tensor:
     """Sum of squares of the interiors."""
     h = halo
     xs = tuple(xs)
-    if xs and h >= 1 and _plain(xs) and all(
+    # (kernels are launched on the current device: tensors of another one go to torch's operations)
+    if xs and h >= 1 and _plain(xs) and xs[0].get_device() == torch.cuda.current_device() and all(
             x.dim() == 3 and x.dtype in (torch.float32, torch.float64) and x.dtype == xs[0].dtype and x.device == xs[0].device
             and min(x.shape) > 2 * h and min(x.stride()) > 0 for x in xs):
         return _SumSquares.apply(h, *xs)

@@ -187,3 +187,28 @@ def test_other_exchanges_run_unfused(cuda, case):
         assert dx._program(1) is None
         with pytest.raises(TypeError, match="one dtype"):
             AG.diffusion_program(dx, run.dev["a"] + run.dev["b"], 2, ALPHA)
+
+
+def loss_in_torch(xs):
+    return sum((x[1:-1, 1:-1, 1:-1] ** 2).sum() for x in xs)
+
+
+def same_as_torch(xs):
+    """The loss and its gradients against torch's operations. The gradients are the same products;
+    both sums of n squares err by less than n roundings."""
+    loss, expected = AG.interior_loss(xs), loss_in_torch(xs)
+    n, eps = sum(x.numel() for x in xs), torch.finfo(loss.dtype).eps
+    return (abs(loss.item() - expected.item()) <= 2 * n * eps * expected.item()
+            and equal(torch.autograd.grad(loss, xs), torch.autograd.grad(expected, xs)))
+
+
+def test_interior_loss_of_another_device(cuda, monkeypatch):
+    """Tensors that are not the current device's: torch's operations, as always."""
+    xs = [torch.randn((6, 5, 7), dtype=torch.float64, device=cuda, requires_grad=True) for _ in range(2)]
+    assert "SumSquares" in type(AG.interior_loss(xs).grad_fn).__name__
+    assert same_as_torch(xs)
+    with monkeypatch.context() as m:
+        m.setattr(torch.cuda, "current_device", lambda: cuda.index + 1)
+        loss = AG.interior_loss(xs)
+    assert "SumSquares" not in type(loss.grad_fn).__name__
+    assert equal(torch.autograd.grad(loss, xs), torch.autograd.grad(loss_in_torch(xs), xs))
