@@ -29,6 +29,8 @@ from collections import OrderedDict
 from typing import Any, Sequence
 
 import torch
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _capi
 from ._capi import call
@@ -336,10 +338,12 @@ def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], st
 
 def _plain(xs) -> bool:
     """Ordinary CUDA tensors outside every transform and mode that sees torch's own operations
-    (functorch, forward-mode AD, dispatch modes, tracing)."""
+    (functorch, forward-mode AD, function and dispatch modes, tracing; a default device is no such
+    mode: it acts on new tensors only)."""
     return (all(type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.layout == torch.strided and not x.is_neg()
                 and not torch._C._functorch.is_functorch_wrapped_tensor(x) for x in xs)
             and torch.autograd.forward_ad._current_level < 0 and torch._C._len_torch_dispatch_stack() == 0
+            and all(type(m) is DeviceContext for m in _get_current_function_mode_stack())
             and not torch.compiler.is_compiling() and not torch.jit.is_tracing())
 
 

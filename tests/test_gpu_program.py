@@ -212,3 +212,22 @@ def test_interior_loss_of_another_device(cuda, monkeypatch):
         loss = AG.interior_loss(xs)
     assert "SumSquares" not in type(loss.grad_fn).__name__
     assert equal(torch.autograd.grad(loss, xs), torch.autograd.grad(loss_in_torch(xs), xs))
+
+
+def test_interior_loss_under_a_function_mode(cuda):
+    """A torch function mode sees the loss's operations; a default device does not change them."""
+    class Names(torch.overrides.TorchFunctionMode):
+        def __init__(self):
+            super().__init__()
+            self.names = []
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            self.names.append(getattr(func, "__name__", ""))
+            return func(*args, **(kwargs or {}))
+    xs = [torch.randn((6, 5, 7), dtype=torch.float64, device=cuda, requires_grad=True)]
+    with Names() as seen:
+        loss = AG.interior_loss(xs)
+    assert any("pow" in name for name in seen.names) and "sum" in seen.names
+    assert equal(torch.autograd.grad(loss, xs), torch.autograd.grad(loss_in_torch(xs), xs))
+    with torch.device(cuda):
+        assert "SumSquares" in type(AG.interior_loss(xs).grad_fn).__name__
