@@ -24,6 +24,7 @@ rewrite of the descriptor tables). Plans hold no references to the tensors they 
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 from collections import OrderedDict
 from typing import Any, Sequence
@@ -222,6 +223,7 @@ def stencil7(xs: Sequence[torch.Tensor], alpha: float = 0.1, halo: int = 1):
     return out if isinstance(out, tuple) else (out,)
 
 
+@functools.lru_cache(maxsize=256)
 def _dense(shape, stride) -> bool:
     """Whether torch.empty_like keeps the strides: the elements fill their memory without gaps or overlaps."""
     n = 1
@@ -373,7 +375,10 @@ class _SumSquares(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         xs, h = ctx.saved_tensors, ctx.halo
-        if torch.is_grad_enabled():  # a gradient that is differentiated in turn: in torch's operations
+        # in torch's operations: a gradient that is differentiated in turn, and gradients of fields
+        # whose strides do not suit new memory (of overlapping elements, as torch.Tensor.unfold's, two
+        # gradients would share one; a slice's gradient would take the whole array's memory)
+        if torch.is_grad_enabled() or not all(_dense(x.shape, x.stride()) for x in xs):
             return (None, *[torch.nn.functional.pad(g * (2 * x[h:-h, h:-h, h:-h]), (h,) * 6) for x in xs])
         dtype, n, ptrs, ext, st = _array_args(xs)
         outs = [torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) for x in xs]

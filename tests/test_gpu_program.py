@@ -231,3 +231,13 @@ def test_interior_loss_under_a_function_mode(cuda):
     assert equal(torch.autograd.grad(loss, xs), torch.autograd.grad(loss_in_torch(xs), xs))
     with torch.device(cuda):
         assert "SumSquares" in type(AG.interior_loss(xs).grad_fn).__name__
+
+
+@pytest.mark.parametrize("strides", ["overlapping", "slice"])
+def test_interior_loss_of_views(cuda, strides):
+    """Fields whose elements share memory, or lie between others': every element has a gradient of its own."""
+    base = torch.randn((10, 8), dtype=torch.float64, device=cuda)
+    x = base.unfold(0, 4, 1) if strides == "overlapping" else torch.randn((12, 9, 14), dtype=torch.float64, device=cuda)[::2, 1:-1, ::2]
+    x = x.detach().requires_grad_(True)
+    assert "SumSquares" in type(AG.interior_loss([x]).grad_fn).__name__
+    assert same_as_torch([x])
