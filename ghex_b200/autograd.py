@@ -340,10 +340,11 @@ def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], st
 
 def _plain(xs) -> bool:
     """Ordinary CUDA tensors outside every transform and mode that sees torch's own operations
-    (functorch, forward-mode AD, function and dispatch modes, tracing; a default device is no such
-    mode: it acts on new tensors only)."""
+    (functorch, batched gradients, forward-mode AD, function and dispatch modes, tracing; a default
+    device is no such mode: it acts on new tensors only)."""
+    functorch = torch._C._functorch
     return (all(type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.layout == torch.strided and not x.is_neg()
-                and not torch._C._functorch.is_functorch_wrapped_tensor(x) for x in xs)
+                and not functorch.is_functorch_wrapped_tensor(x) and not functorch.is_legacy_batchedtensor(x) for x in xs)
             and torch.autograd.forward_ad._current_level < 0 and torch._C._len_torch_dispatch_stack() == 0
             and all(type(m) is DeviceContext for m in _get_current_function_mode_stack())
             and not torch.compiler.is_compiling() and not torch.jit.is_tracing())
@@ -375,10 +376,11 @@ class _SumSquares(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         xs, h = ctx.saved_tensors, ctx.halo
-        # in torch's operations: a gradient that is differentiated in turn, and gradients of fields
-        # whose strides do not suit new memory (of overlapping elements, as torch.Tensor.unfold's, two
-        # gradients would share one; a slice's gradient would take the whole array's memory)
-        if torch.is_grad_enabled() or not all(_dense(x.shape, x.stride()) for x in xs):
+        # in torch's operations: a gradient that is differentiated in turn, or batched (vmap), and
+        # gradients of fields whose strides do not suit new memory (of overlapping elements, as
+        # torch.Tensor.unfold's, two gradients would share one; a slice's gradient would take the
+        # whole array's memory)
+        if torch.is_grad_enabled() or not _plain((g, *xs)) or not all(_dense(x.shape, x.stride()) for x in xs):
             return (None, *[torch.nn.functional.pad(g * (2 * x[h:-h, h:-h, h:-h]), (h,) * 6) for x in xs])
         dtype, n, ptrs, ext, st = _array_args(xs)
         outs = [torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) for x in xs]

@@ -241,3 +241,10 @@ def test_interior_loss_of_views(cuda, strides):
     x = x.detach().requires_grad_(True)
     assert "SumSquares" in type(AG.interior_loss([x]).grad_fn).__name__
     assert same_as_torch([x])
+
+
+def test_interior_loss_with_a_batched_gradient(cuda):
+    xs = [torch.randn((6, 5, 7), dtype=torch.float64, device=cuda, requires_grad=True) for _ in range(2)]
+    seeds = torch.tensor([1.0, -0.5, 3.0], dtype=torch.float64, device=cuda)
+    got = torch.autograd.grad(AG.interior_loss(xs), xs, seeds, is_grads_batched=True)
+    assert equal(got, torch.autograd.grad(loss_in_torch(xs), xs, seeds, is_grads_batched=True))
