@@ -376,11 +376,12 @@ class _SumSquares(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         xs, h = ctx.saved_tensors, ctx.halo
-        # in torch's operations: a gradient that is differentiated in turn, or batched (vmap), and
-        # gradients of fields whose strides do not suit new memory (of overlapping elements, as
-        # torch.Tensor.unfold's, two gradients would share one; a slice's gradient would take the
-        # whole array's memory)
-        if torch.is_grad_enabled() or not _plain((g, *xs)) or not all(_dense(x.shape, x.stride()) for x in xs):
+        # in torch's operations: a gradient that is differentiated in turn, or batched (vmap); fields
+        # that a saved-tensor hook gave back as something else; and gradients of fields whose
+        # strides do not suit new memory (of overlapping elements, as torch.Tensor.unfold's, two
+        # gradients would share one; a slice's gradient would take the whole array's memory)
+        if torch.is_grad_enabled() or not _plain((g, *xs)) or not all(
+                x.dtype == g.dtype and x.device == g.device and _dense(x.shape, x.stride()) for x in xs):
             return (None, *[torch.nn.functional.pad(g * (2 * x[h:-h, h:-h, h:-h]), (h,) * 6) for x in xs])
         dtype, n, ptrs, ext, st = _array_args(xs)
         outs = [torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device) for x in xs]

@@ -248,3 +248,16 @@ def test_interior_loss_with_a_batched_gradient(cuda):
     seeds = torch.tensor([1.0, -0.5, 3.0], dtype=torch.float64, device=cuda)
     got = torch.autograd.grad(AG.interior_loss(xs), xs, seeds, is_grads_batched=True)
     assert equal(got, torch.autograd.grad(loss_in_torch(xs), xs, seeds, is_grads_batched=True))
+
+
+def test_interior_loss_of_unpacked_tensors(cuda):
+    """A saved-tensor hook that keeps the fields in single precision: the gradient is that of the
+    fields as they were kept. One that gives them back contiguous: the gradient is the same."""
+    x = torch.randn((7, 5, 6), dtype=torch.float64, device=cuda).permute(2, 1, 0).requires_grad_(True)
+    for pack, kept in ((lambda t: t.float(), x.detach().float().double()), (lambda t: t.contiguous(), x.detach())):
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+            loss = AG.interior_loss([x])
+        (g,) = torch.autograd.grad(loss, [x])
+        expected = torch.zeros_like(x)
+        expected[1:-1, 1:-1, 1:-1] = 2 * kept[1:-1, 1:-1, 1:-1]
+        assert equal([g], [expected])
