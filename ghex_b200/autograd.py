@@ -328,7 +328,9 @@ def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], st
     writes into xs: pass clones of leaf tensors that require grad. Where the exchange allows it,
     a step is one kernel (same bits)."""
     xs = tuple(xs)
-    if steps > 0 and type(dx) is DifferentiableExchange and math.isfinite(alpha):
+    # (a function that changes a view in place may have one output only: a single field's exchange)
+    view = torch.is_grad_enabled() and any(isinstance(x, torch.Tensor) and x.requires_grad and x._is_view() for x in xs)
+    if steps > 0 and type(dx) is DifferentiableExchange and math.isfinite(alpha) and not view:
         program = dx._program(halo)
         if program is not None:
             return _Diffusion.apply(dx, program, steps, alpha, halo, *xs)[len(xs):]

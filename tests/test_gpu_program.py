@@ -164,6 +164,18 @@ def test_interior_loss_is_differentiable_twice(cuda):
     assert bits_equal(gg.cpu().numpy(), expected.cpu().numpy()) == 0
 
 
+def test_single_field_that_is_a_view(cuda):
+    """One periodic domain whose field is a view in a graph: an exchange in place with one output."""
+    dx, x0 = make(cuda, (9, 8, 6), (1, 1, 1), (True, True, True), 1, np.float64, None)
+    assert dx._program(1) is not None
+    results = []
+    for program in (lambda x: AG.diffusion_program(dx, [x], 3, ALPHA), lambda x: separately(dx, [x], 3, 1)[1]):
+        leaf = x0[0].clone().requires_grad_(True)
+        (y,) = program(leaf.clone()[:])
+        results.append([y, *torch.autograd.grad((y * y).sum(), [leaf])])
+    assert equal(*results)
+
+
 @pytest.mark.parametrize("case", ["halo", "thin", "fields of two types"])
 def test_other_exchanges_run_unfused(cuda, case):
     """A pattern halo wider than the update's, domains one cell thick, fields of two types: the
