@@ -122,6 +122,11 @@ class DifferentiableExchange:
         stream = torch.cuda.current_stream(grads[0].device)
         self._bwd.get(grads, stream).adjoint(stream=stream)
 
+    def _finite(self, alpha: float) -> bool:
+        """Whether alpha is finite in the fields' type: only then is the gradient of a halo cell that
+        no interior cell lies beside zero, and the program may leave it out."""
+        return math.isfinite(C.c_float(alpha).value if self._tensor_layout[0][2] == torch.float32 else alpha)
+
     def _program(self, halo: int):
         """The exchange and the 7-point update in fused passes, or None for an exchange that
         ghexb_program_create refuses (then the two run one after the other)."""
@@ -330,7 +335,7 @@ def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], st
     xs = tuple(xs)
     # (a function that changes a view in place may have one output only: a single field's exchange)
     view = torch.is_grad_enabled() and any(isinstance(x, torch.Tensor) and x.requires_grad and x._is_view() for x in xs)
-    if steps > 0 and type(dx) is DifferentiableExchange and math.isfinite(alpha) and not view:
+    if steps > 0 and type(dx) is DifferentiableExchange and dx._finite(alpha) and not view:
         program = dx._program(halo)
         if program is not None:
             return _Diffusion.apply(dx, program, steps, alpha, halo, *xs)[len(xs):]
@@ -425,7 +430,7 @@ class GraphedDiffusion:
         dx.check(templates)
         self.dx, self.steps, self.alpha, self.halo = dx, steps, alpha, halo
         dev = templates[0].device
-        self._program = dx._program(halo) if steps > 0 and math.isfinite(alpha) else None
+        self._program = dx._program(halo) if steps > 0 and dx._finite(alpha) else None
         if self._program is not None:
             self._capture_fused(templates, dev)
             return

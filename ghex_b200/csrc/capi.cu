@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -1099,6 +1100,7 @@ int ghexb_program_steps(ghexb_program program, const void* const* fields, const 
     return guarded([&] {
         require(program != nullptr, "null argument");
         require(steps >= 1, "a program runs at least one step");
+        require(std::isfinite(program->f64 ? alpha : (double)(float)alpha), "an alpha that is not finite in the fields' type");
         require((fields != nullptr) != (source != nullptr), "either the fields or a packed source is needed");
         require(!twice || (adjoint && source), "only a packed source of the transpose is doubled");
         const size_t n = program->domains.size(), es = program->f64 ? 8 : 4;

@@ -13,6 +13,7 @@ import torch
 
 from ghex_b200 import autograd as AG
 from ghex_b200 import workloads as W
+from ghex_b200._capi import GhexError
 
 from gpu_helpers import RegularRun, bits_equal
 
@@ -162,6 +163,26 @@ def test_interior_loss_is_differentiable_twice(cuda):
     expected = torch.zeros_like(x)
     expected[1:-1, 1:-1, 1:-1] = 8 * x.detach()[1:-1, 1:-1, 1:-1]
     assert bits_equal(gg.cpu().numpy(), expected.cpu().numpy()) == 0
+
+
+@pytest.mark.parametrize("alpha", [1e39, float("inf")])
+def test_alpha_beyond_the_fields_type(cuda, alpha):
+    """An alpha that is infinite in single precision: the gradients of halo edges are not zero then
+    (infinity times zero), and reach the cells they were copied from."""
+    dx, x0 = make(cuda, (12, 10, 8), (2, 1, 1), (True, True, True), 1, np.float32, None)
+    weights = [x.abs() ** 4 + 1e-3 for x in x0]  # positive, some far below their neighbours: infinite with one sign
+    results = []
+    for fused in (False, True):
+        leaves = [x.clone().requires_grad_(True) for x in x0]
+        xs = [x.clone() for x in leaves]
+        if fused:
+            ys = AG.diffusion_program(dx, xs, 1, alpha)
+        else:
+            ys = AG.stencil7(dx(*xs), alpha)
+        results.append([torch.isnan(t) for t in (*ys, *torch.autograd.grad(ys, leaves, weights))])
+    assert all(bool((a == b).all()) for a, b in zip(*results))
+    with pytest.raises(GhexError, match="finite"):
+        dx._program(1).steps(1, alpha, torch.cuda.current_stream(), fields=x0, out=[torch.empty_like(x) for x in x0])
 
 
 def test_single_field_that_is_a_view(cuda):
