@@ -26,6 +26,7 @@ from __future__ import annotations
 import ctypes as C
 import functools
 import math
+import operator
 from collections import OrderedDict
 from typing import Any, Sequence
 
@@ -332,7 +333,7 @@ def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], st
     """steps x (halo exchange, 7-point update); returns the final fields. The first exchange
     writes into xs: pass clones of leaf tensors that require grad. Where the exchange allows it,
     a step is one kernel (same bits)."""
-    xs = tuple(xs)
+    xs, steps = tuple(xs), operator.index(steps)
     # (a function that changes a view in place may have one output only: a single field's exchange)
     view = torch.is_grad_enabled() and any(isinstance(x, torch.Tensor) and x.requires_grad and x._is_view() for x in xs)
     if steps > 0 and type(dx) is DifferentiableExchange and dx._finite(alpha) and not view:
@@ -428,6 +429,7 @@ class GraphedDiffusion:
                  alpha: float = 0.1, halo: int = 1):
         templates = list(templates)
         dx.check(templates)
+        steps = operator.index(steps)
         self.dx, self.steps, self.alpha, self.halo = dx, steps, alpha, halo
         dev = templates[0].device
         self._program = dx._program(halo) if steps > 0 and dx._finite(alpha) else None

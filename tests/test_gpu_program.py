@@ -197,6 +197,17 @@ def test_single_field_that_is_a_view(cuda):
     assert equal(*results)
 
 
+def test_steps_are_whole_numbers(cuda):
+    """Any index counts steps; a float is refused before the inputs are touched."""
+    dx, x0 = make(cuda, (12, 10, 8), (2, 1, 1), (True, True, True), 1, np.float64, None)
+    xs = [x.clone() for x in x0]
+    for program in (AG.diffusion_program, AG.GraphedDiffusion):
+        with pytest.raises(TypeError):
+            program(dx, xs, 2.0, ALPHA)
+    assert equal(xs, x0)
+    assert equal(AG.diffusion_program(dx, [x.clone() for x in x0], np.int64(2), ALPHA), separately(dx, xs, 2, 1)[1])
+
+
 @pytest.mark.parametrize("case", ["halo", "thin", "fields of two types"])
 def test_other_exchanges_run_unfused(cuda, case):
     """A pattern halo wider than the update's, domains one cell thick, fields of two types: the
