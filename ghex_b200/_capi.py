@@ -150,6 +150,7 @@ SIGNATURES = {
     "ghexb_program_create": [C.POINTER(_vp), _i, _i, C.POINTER(_vp)],
     "ghexb_program_destroy": [_vp],
     "ghexb_program_status": [_vp, C.POINTER(C.c_uint)],
+    "ghexb_program_status_word": [_vp, C.POINTER(C.POINTER(C.c_uint))],
     "ghexb_program_buffer_bytes": [_vp, _pi64],
     "ghexb_program_steps": [_vp, C.POINTER(_vp), _vp, C.POINTER(_vp), _vp, _vp, _i, C.c_double, _i, _i, _vp],
     "ghexb_sumsq_partials": [_i, _i, _pi64, _i, _pi64],

@@ -266,7 +266,8 @@ class _Program:
              float(alpha), int(adjoint), int(twice), C.c_void_p(stream.cuda_stream))
 
     def status(self) -> int:
-        """The passes' status word since the last call (0: every load arrived in time)."""
+        """The passes' status word since it was last looked at, after a wait for the device (0: every
+        load arrived in time). steps() looks at it as well, without a wait."""
         v = C.c_uint()
         call("ghexb_program_status", self._h, C.byref(v))
         return v.value
@@ -332,7 +333,8 @@ def diffusion_program(dx: DifferentiableExchange, xs: Sequence[torch.Tensor], st
                       halo: int = 1):
     """steps x (halo exchange, 7-point update); returns the final fields. The first exchange
     writes into xs: pass clones of leaf tensors that require grad. Where the exchange allows it,
-    a step is one kernel (same bits)."""
+    a step is one kernel (same bits). Should a kernel's load not arrive within a second, the cells
+    that depend on it are not numbers, and the next program on this exchange raises GhexError."""
     xs, steps = tuple(xs), operator.index(steps)
     # (a function that changes a view in place may have one output only: a single field's exchange)
     view = torch.is_grad_enabled() and any(isinstance(x, torch.Tensor) and x.requires_grad and x._is_view() for x in xs)
@@ -423,7 +425,8 @@ class GraphedDiffusion:
     buffer sets; the backward seeds 2 x (final interior) and applies, for every step in reverse, the
     stencil's transpose and then the exchange's adjoint, on two more buffer sets, with four exchange
     plans of its own bound to the four sets before the capture. ``run(xs)`` returns the loss and
-    the gradient (tensors the next run overwrites)."""
+    the gradient (tensors the next run overwrites); a load that does not arrive is seen as by
+    ``diffusion_program``."""
 
     def __init__(self, dx: DifferentiableExchange, templates: Sequence[torch.Tensor], steps: int = 10,
                  alpha: float = 0.1, halo: int = 1):

@@ -1057,6 +1057,12 @@ int ghexb_stencil7(int dtype, int n, const void* const* in, void* const* out, co
 }
 
 // ---- the program in fused passes -------------------------------------------------------------
+namespace
+{
+// the status word as the device has left it so far, and none from here on
+unsigned take_status(ghexb_program_s& program) { return __atomic_exchange_n(program.status, 0u, __ATOMIC_ACQ_REL); }
+} // namespace
+
 int ghexb_program_create(const ghexb_field* fields, int n, int halo, ghexb_program* out)
 {
     return guarded([&] {
@@ -1065,8 +1071,7 @@ int ghexb_program_create(const ghexb_field* fields, int n, int halo, ghexb_progr
         for (int i = 0; i < n; ++i) require(fields[i] != nullptr, "null field handle");
         auto p = std::make_unique<ghexb_program_s>();
         ghexb::build_program(*p, fields, n, halo);
-        ghexb::check_cuda(cudaMalloc(&p->status, sizeof(unsigned)), "cudaMalloc(program status)");
-        ghexb::check_cuda(cudaMemset(p->status, 0, sizeof(unsigned)), "cudaMemset(program status)");
+        p->status = ghexb::take_status_word();
         *out = p.release();
     });
 }
@@ -1075,8 +1080,16 @@ int ghexb_program_status(ghexb_program program, unsigned* status)
 {
     return guarded([&] {
         require(program && status, "null argument");
-        ghexb::check_cuda(cudaMemcpy(status, program->status, sizeof(unsigned), cudaMemcpyDeviceToHost), "cudaMemcpy(program status)");
-        ghexb::check_cuda(cudaMemset(program->status, 0, sizeof(unsigned)), "cudaMemset(program status)");
+        ghexb::check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize(program status)");
+        *status = take_status(*program);
+    });
+}
+
+int ghexb_program_status_word(ghexb_program program, unsigned** word)
+{
+    return guarded([&] {
+        require(program && word, "null argument");
+        *word = program->status;
     });
 }
 
@@ -1116,6 +1129,8 @@ int ghexb_program_steps(ghexb_program program, const void* const* fields, const 
         require(packed < 1 || ((source == a ? b : a) != nullptr), "a packed buffer is missing");
         require(packed < 2 || (a && b && a != b), "two packed buffers are needed");
         require(aligned(a, 16) && aligned(b, 16) && aligned(source, 16), "packed buffers are 16-byte aligned");
+        if (take_status(*program))
+            throw ghexb::error(GHEXB_ERR_INTERNAL, "a load of an earlier pass of this program did not arrive in time: its results are not numbers");
         ghexb::check_cuda(ghexb::launch_passes(*program, fields, source, out, a, b, steps, alpha, adjoint != 0, twice != 0,
                               static_cast<cudaStream_t>(stream)),
             "program launch");

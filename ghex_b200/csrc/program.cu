@@ -21,10 +21,12 @@
 
 #include <algorithm>
 #include <map>
+#include <mutex>
 #include <string>
 #include <utility>
 
 #include "async_copy.hpp"
+#include "plan.hpp"
 #include "program.hpp"
 #include "staged.hpp"
 
@@ -120,6 +122,15 @@ template <typename T> __device__ __forceinline__ cells<T> zero_if(bool z, const 
     for (int v = 0; v < cells<T>::V; ++v) c.v[v] = z ? T(0) : a.v[v];
     return c;
 }
+
+template <typename T> __device__ __forceinline__ void not_a_number(cells<T>& a)
+{
+#pragma unroll
+    for (int v = 0; v < cells<T>::V; ++v) a.v[v] = sizeof(T) == 8 ? (T)__longlong_as_double(0x7ff8000000000000ll) : (T)__int_as_float(0x7fc00000);
+}
+
+// the program's status word (host memory)
+__device__ __forceinline__ void report(unsigned* status) { *reinterpret_cast<volatile unsigned*>(status) = 1u; }
 
 constexpr int k_batch = 32; // domains per launch
 
@@ -598,7 +609,7 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
                 const int st = q % S;
                 ok = q < S || mbar_wait(&empty[st], (uint32_t)(q / S - 1) & 1u);
                 if (ok) issue(q, st);
-                else atomicOr(args.status, 1u);
+                else report(args.status);
             }
             // the block's shared memory is not given back before its last loads have landed (the
             // other threads wait for every plane; this is for those that gave up)
@@ -624,12 +635,14 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
         }
         copy_commit();
     };
-    bool failed = false; // a load did not arrive in time: nothing more is waited for or stored
+    // a load did not arrive in time: nothing more is waited for, and what depends on it is not a
+    // number, here and in every result computed from it
+    bool failed = false;
     const auto wait = [&](int st, uint32_t parity) {
         if (!failed && !mbar_wait(&full[st], parity))
         {
             failed = true;
-            atomicOr(args.status, 1u);
+            report(args.status);
         }
     };
 #pragma unroll
@@ -732,7 +745,12 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
                 }
             }
         }
-        if (live && !failed)
+        if (failed)
+        {
+#pragma unroll
+            for (int r = 0; r < R; ++r) not_a_number(y[r]);
+        }
+        if (live)
         {
 #pragma unroll
             for (int r = 0; r < R; ++r)
@@ -1001,6 +1019,53 @@ cudaError_t launch_passes(const ghexb_program_s& P, const void* const* fields, c
                  : launch_passes_any<float>(P, fields, source, out, a, b, steps, alpha, adjoint, twice, stream);
 }
 
+// ---- status words ------------------------------------------------------------------------------
+namespace
+{
+struct status_words
+{
+    std::mutex mutex;
+    std::vector<unsigned*> unused; // each one address on the host and on every device
+};
+status_words& statuses()
+{
+    static status_words& words = *new status_words; // programs may outlive the library's statics
+    return words;
+}
+} // namespace
+
+unsigned* take_status_word()
+{
+    constexpr int count = 1024;
+    status_words& s = statuses();
+    std::lock_guard<std::mutex> lock(s.mutex);
+    if (s.unused.empty())
+    {
+        void* p = nullptr;
+        check_cuda(cudaHostAlloc(&p, count * sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc(program status)");
+        for (int i = count; i-- > 0;) s.unused.push_back(static_cast<unsigned*>(p) + i);
+    }
+    unsigned* word = s.unused.back();
+    s.unused.pop_back();
+    *word = 0;
+    return word;
+}
+
+void return_status_word(unsigned* word)
+{
+    status_words& s = statuses();
+    std::lock_guard<std::mutex> lock(s.mutex);
+    s.unused.push_back(word);
+}
+} // namespace ghexb
+
+ghexb_program_s::~ghexb_program_s()
+{
+    if (status) ghexb::return_status_word(status);
+}
+
+namespace ghexb
+{
 // ---- geometry ----------------------------------------------------------------------------------
 void build_program(ghexb_program_s& P, const ghexb_field* fields, int nfields, int halo)
 {

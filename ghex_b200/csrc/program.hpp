@@ -31,17 +31,22 @@ struct ghexb_program_s
     int32_t halo = 1;
     int64_t packed_elements = 0;
     std::vector<ghexb::program_domain> domains; // one per field
-    // device word: bit 0, a load of a pass did not arrive in time (its outputs are not written)
+    // page-locked host word that the passes write and the host reads without waiting: 1, a load of a
+    // pass did not arrive in time (what depended on it is not a number)
     unsigned* status = nullptr;
 
-    ~ghexb_program_s()
-    {
-        if (status) cudaFree(status);
-    }
+    ~ghexb_program_s();
 };
 
 namespace ghexb
 {
+// Status words (0 when taken), shared out by all programs from pages of 1024: page-locking one for
+// each took 1 to 7 ms, as much as the rest of a graphed program's set-up (4.2 ms for 500 x 510 x 250;
+// 5.5 to 7 with a word allocated on the device each). A page stays until the process ends, its words
+// are used again.
+unsigned* take_status_word();
+void return_status_word(unsigned* word);
+
 // The program's geometry from the fields of an exchange (n >= 1; their memory is not kept): every
 // halo region must be written whole by the exchange or not at all, and every face of a domain must
 // be a whole face of one neighbour. Throws ghexb::error (GHEXB_ERR_INVALID, with the reason) for

@@ -389,9 +389,13 @@ int ghexb_stencil7(int dtype, int n, const void* const* in, void* const* out, co
  * GHEXB_ERR_INVALID. The fields' memory is not kept. */
 int ghexb_program_create(const ghexb_field* fields, int n, int halo, ghexb_program* out);
 int ghexb_program_destroy(ghexb_program program);
-/* The program's status word since the last call: 0, or bit 0 when a load of a pass did not arrive
- * in time (about a second; the pass ended without writing what depended on it). */
+/* The program's status word since it was last looked at, after a wait for the device: 0, or bit 0
+ * when a load of a pass did not arrive in time (about a second; what depended on it, in this pass
+ * and those after it, is not a number). ghexb_program_steps looks at it too, without a wait, and
+ * fails once with GHEXB_ERR_INTERNAL when an earlier pass has left it set. */
 int ghexb_program_status(ghexb_program program, unsigned* status);
+/* Where that word is, in page-locked host memory: it may be read at any time. */
+int ghexb_program_status_word(ghexb_program program, unsigned** word);
 /* Size of a packed buffer (16-byte aligned device memory) that holds every interior. */
 int ghexb_program_buffer_bytes(ghexb_program program, int64_t* bytes);
 /* `steps` >= 1 passes. The first reads the caller's fields (fields[i] laid out as the i-th field

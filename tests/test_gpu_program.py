@@ -7,10 +7,13 @@ more domains than one launch takes. Every value is one of the same operations wi
 roundings, so the tolerance is zero."""
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
+from ghex_b200 import _capi
 from ghex_b200 import autograd as AG
 from ghex_b200 import workloads as W
 from ghex_b200._capi import GhexError
@@ -305,3 +308,21 @@ def test_interior_loss_of_unpacked_tensors(cuda):
         expected = torch.zeros_like(x)
         expected[1:-1, 1:-1, 1:-1] = 2 * kept[1:-1, 1:-1, 1:-1]
         assert equal([g], [expected])
+
+
+def test_a_pass_that_gave_up_is_reported(cuda):
+    """The status word as a kernel leaves it when a load does not arrive, written by the host: the
+    next program of the exchange raises, once, and then runs."""
+    dx, x0 = make(cuda, (12, 10, 8), (2, 1, 1), (True, True, True), 1, np.float64, None)
+    graphed = AG.GraphedDiffusion(dx, x0, 2, ALPHA)
+    word = C.POINTER(C.c_uint)()
+    _capi.call("ghexb_program_status_word", dx._program(1)._h, C.byref(word))
+    _, ys = separately(dx, [x.clone() for x in x0], 2, 1)
+    for program in (lambda: AG.diffusion_program(dx, [x.clone() for x in x0], 2, ALPHA), lambda: graphed.run(x0)):
+        word[0] = 1
+        with pytest.raises(GhexError, match="did not arrive in time"):
+            program()
+        program()
+    assert equal(AG.diffusion_program(dx, [x.clone() for x in x0], 2, ALPHA), ys)
+    word[0] = 1
+    assert dx._program(1).status() == 1 and dx._program(1).status() == 0
