@@ -603,17 +603,20 @@ __global__ void __launch_bounds__(k_tile_threads + 32, k_tile_resident) tile_ker
     {
         if (threadIdx.x == k_tile_threads)
         {
-            bool ok = true;
-            for (int q = 0; q < planes && ok; ++q)
+            int issued = 0;
+            for (; issued < planes; ++issued)
             {
-                const int st = q % S;
-                ok = q < S || mbar_wait(&empty[st], (uint32_t)(q / S - 1) & 1u);
-                if (ok) issue(q, st);
-                else report(args.status);
+                const int st = issued % S;
+                if (issued >= S && !mbar_wait(&empty[st], (uint32_t)(issued / S - 1) & 1u))
+                {
+                    report(args.status);
+                    break;
+                }
+                issue(issued, st);
             }
-            // the block's shared memory is not given back before its last loads have landed (the
-            // other threads wait for every plane; this is for those that gave up)
-            for (int q = max(0, planes - S); q < planes && ok; ++q) ok = mbar_wait(&full[q % S], (uint32_t)(q / S) & 1u);
+            // the block's shared memory is not given back before its last loads have landed, also where
+            // the stages ran out or the other threads gave up
+            for (int q = max(0, issued - S); q < issued; ++q) mbar_wait(&full[q % S], (uint32_t)(q / S) & 1u);
         }
         return;
     }
