@@ -141,6 +141,8 @@ constexpr int k_batch = 32; // domains per launch
 // -> 90.5. Let go at a block's start instead, the next pass's blocks settle in whatever slots are
 // free and leave some SMs with more of them than others: 330 and 101.7 us, and 64 x 200 x 60 157 us
 // where it had been 148 (at the last plane: 145).
+// What the pass before wrote is read by ordinary loads: it is not constant while the kernel runs, so
+// neither __ldg nor a const __restrict__ pointer may name it.
 __device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void lead() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Params, typename... Args>
@@ -216,7 +218,7 @@ __device__ __forceinline__ void write_halo(const pass_domain& d, T alpha, uint32
     const int h = d.halo, nx = d.nx, ny = d.ny, nz = d.nz;
     const uint32_t ex = nx + 2 * h, ey = ny + 2 * h;
     const uint32_t zcells = ex * ey * (2 * h), ycells = ex * (2 * h) * nz, xcells = (2 * h) * ny * nz;
-    const T* __restrict__ in = static_cast<const T*>(d.in);
+    const T* in = static_cast<const T*>(d.in);
     T* __restrict__ out = static_cast<T*>(d.out);
     for (int q = 0; q < k_halo_cells; ++q)
     {
@@ -251,7 +253,7 @@ __device__ __forceinline__ void write_halo(const pass_domain& d, T alpha, uint32
             {
                 const auto G = [&](int a, int b, int e) {
                     if (a < 0 || a >= nx || b < 0 || b >= ny || e < 0 || e >= nz) return T(0);
-                    const T g = __ldg(in + (a * d.isx + b * d.isy + e * d.isz));
+                    const T g = in[a * d.isx + b * d.isy + e * d.isz];
                     return TWICE ? mul_rn(T(2), g) : g;
                 };
                 T t = add_rn(G(i - 1, j, k), G(i + 1, j, k));
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(k_threads, k_resident) pass_kernel(const __gri
     const int k0 = (int)(bz * d.slab), k1 = min(nz, k0 + (int)d.slab);
     const int i0 = (int)(column - strip * d.chunks) * V, m = min(V, nx - i0);
     const int j0 = min((int)strip * R, ny - R); // the last strip overlaps the one before (same values)
-    const T* __restrict__ in = static_cast<const T*>(d.in);
+    const T* in = static_cast<const T*>(d.in);
     T* __restrict__ out = static_cast<T*>(d.out);
     const int sx = d.isx, sy = d.isy, sz = d.isz;
     const bool first = i0 == 0, last = i0 + V >= nx; // the chunk touches face x-, x+
@@ -1204,7 +1206,7 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_kernel(const __grid_const
     b -= d.block0;
     follow();
     const uint64_t all = (uint64_t)d.chunks * d.ny * d.nz;
-    const T* __restrict__ p = static_cast<const T*>(d.p);
+    const T* p = static_cast<const T*>(d.p);
     cells<T> c[k_sum_chunks];
     int m[k_sum_chunks];
 #pragma unroll
@@ -1223,13 +1225,13 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_kernel(const __grid_const
                 int4 w;
                 cells<T> c;
             } u;
-            u.w = __ldg(reinterpret_cast<const int4*>(p + (i0 + j * d.sy + k * d.sz)));
+            u.w = *reinterpret_cast<const int4*>(p + (i0 + j * d.sy + k * d.sz));
             c[q] = u.c;
         }
         else
         {
 #pragma unroll
-            for (int v = 0; v < V; ++v) c[q].v[v] = v < m[q] ? __ldg(p + ((int64_t)(i0 + v) * d.sx + j * d.sy + k * d.sz)) : T(0);
+            for (int v = 0; v < V; ++v) c[q].v[v] = v < m[q] ? p[(int64_t)(i0 + v) * d.sx + j * d.sy + k * d.sz] : T(0);
         }
     }
     double s = 0;
@@ -1242,7 +1244,7 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_kernel(const __grid_const
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
-template <typename T> __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* __restrict__ partials, uint32_t n, T* out)
+template <typename T> __global__ void __launch_bounds__(1024) sum_partials_kernel(const double* partials, uint32_t n, T* out)
 {
     follow();
     double s = 0;
@@ -1266,7 +1268,7 @@ struct grad_args
 };
 
 template <typename T>
-__global__ void __launch_bounds__(k_sum_threads) sumsq_grad_kernel(const __grid_constant__ grad_args args, const T* __restrict__ g)
+__global__ void __launch_bounds__(k_sum_threads) sumsq_grad_kernel(const __grid_constant__ grad_args args, const T* g)
 {
     uint32_t b = blockIdx.x;
     int di = 0;
@@ -1276,27 +1278,29 @@ __global__ void __launch_bounds__(k_sum_threads) sumsq_grad_kernel(const __grid_
     const int h = args.halo;
     follow();
     const uint64_t all = (uint64_t)d.ex * d.ey * d.ez;
-    const T scale = __ldg(g);
-    const T* __restrict__ p = static_cast<const T*>(d.p);
+    const T scale = *g;
+    const T* p = static_cast<const T*>(d.p);
     T* __restrict__ out = static_cast<T*>(d.out);
     T x[k_sum_chunks];
     int64_t at[k_sum_chunks];
+    bool inside[k_sum_chunks];
 #pragma unroll
     for (int q = 0; q < k_sum_chunks; ++q)
     {
         const uint64_t e = ((uint64_t)b * k_sum_chunks + q) * k_sum_threads + threadIdx.x;
         at[q] = -1;
-        x[q] = T(0);
+        x[q] = T(0), inside[q] = false;
         if (e >= all) continue;
         const uint32_t row = all >> 31 ? (uint32_t)(e / d.ex) : d.by_row.div((uint32_t)e);
         const int i = (int)(e - (uint64_t)row * d.ex), k = (int)d.by_rows.div(row), j = (int)(row - (uint32_t)k * d.ey);
         at[q] = (int64_t)i * d.sx + (int64_t)j * d.sy + (int64_t)k * d.sz;
-        if (i >= h && i < d.ex - h && j >= h && j < d.ey - h && k >= h && k < d.ez - h)
-            x[q] = mul_rn(scale, mul_rn(T(2), __ldg(p + at[q])));
+        inside[q] = i >= h && i < d.ex - h && j >= h && j < d.ey - h && k >= h && k < d.ez - h;
+        if (inside[q]) x[q] = p[at[q]];
     }
+    // (products in a loop of their own: every load is under way before the first is waited for)
 #pragma unroll
     for (int q = 0; q < k_sum_chunks; ++q)
-        if (at[q] >= 0) out[at[q]] = x[q];
+        if (at[q] >= 0) out[at[q]] = inside[q] ? mul_rn(scale, mul_rn(T(2), x[q])) : T(0);
 }
 
 uint64_t sum_blocks(int V, const int32_t* n)
