@@ -1222,6 +1222,46 @@ void check_relocation(ghexb_plan_s& plan)
     if (!equal) throw error(GHEXB_ERR_INTERNAL, "moved tile tables differ from the tables built at the new address");
 }
 
+namespace
+{
+// Column and level of element e of a list tile, as exchange.cu decomposes it.
+std::pair<uint32_t, uint32_t> list_element(const xtile& t, uint32_t e)
+{
+    if (t.n1 > 1)
+    {
+        const uint32_t lev = fast_div{t.n1, t.m1, t.l1}.div(e);
+        return {(uint32_t)t.u0 + (e - lev * t.n1), lev};
+    }
+    const uint32_t g = t.e0 + e, col = fast_div{t.n0, t.m0, t.l0}.div(g);
+    return {col, g - col * t.n0};
+}
+
+// Owner and level of element e of an unstructured gather tile.
+std::pair<uint32_t, uint32_t> list_element(const gtile& t, uint32_t e)
+{
+    if (t.n1 > 1)
+    {
+        const uint32_t lev = fast_div{t.n1, t.m1, t.l1}.div(e);
+        return {fast_div{t.n0, t.m0, t.l0}.div(t.e0) + (e - lev * t.n1), lev};
+    }
+    const uint32_t g = t.e0 + e, own = fast_div{t.n0, t.m0, t.l0}.div(g);
+    return {own, g - own * t.n0};
+}
+
+// A tile's elements are those from e0 on of columns of n0 levels, each once, in whichever order.
+template <typename Tile> void check_list_elements(const Tile& t)
+{
+    std::vector<char> seen(t.count, 0);
+    for (uint32_t e = 0; e < t.count; ++e)
+    {
+        const auto [col, lev] = list_element(t, e);
+        const uint64_t at = (uint64_t)col * t.n0 + lev;
+        if (lev >= t.n0 || at < t.e0 || at - t.e0 >= t.count || seen[at - t.e0]++)
+            throw error(GHEXB_ERR_INTERNAL, "list element decomposition out of range");
+    }
+}
+} // namespace
+
 int64_t check_tables(ghexb_plan_s& plan)
 {
     build_tiles(plan, plan.idx.data());
@@ -1230,12 +1270,13 @@ int64_t check_tables(ghexb_plan_s& plan)
     auto replay = [&](const xtile& t, const ghexb_field_s& sf, const ghexb_field_s& df) {
         const int64_t k = t.unit / sf.esize; // elements per unit
         const int64_t ss = field_span(sf), ds = field_span(df);
+        if (t.kind == 1) check_list_elements(t);
         for (uint32_t e = 0; e < t.count; ++e)
         {
-            const uint32_t g = t.e0 + e;
             int64_t so, dof;
             if (t.kind == 0)
             {
+                const uint32_t g = t.e0 + e;
                 const uint32_t r = fast_div{t.n0, t.m0, t.l0}.div(g);
                 const int64_t i0 = g - r * t.n0;
                 const uint32_t i2 = fast_div{t.n1, t.m1, t.l1}.div(r);
@@ -1247,8 +1288,8 @@ int64_t check_tables(ghexb_plan_s& plan)
             }
             else
             {
-                const uint32_t col = fast_div{t.n0, t.m0, t.l0}.div(g);
-                const int64_t lev = g - col * t.n0;
+                const auto [col, level] = list_element(t, e);
+                const int64_t lev = level;
                 so = (int64_t)t.sidx[col] * t.s0 + lev * t.s1;
                 dof = (int64_t)t.didx[col] * t.d0 + lev * t.d1;
             }
@@ -1270,7 +1311,24 @@ int64_t check_tables(ghexb_plan_s& plan)
     };
     for (size_t i = 0; i < plan.boxes.size(); ++i) replay_range(plan.xb_box[i], plan.box_src_slot[i], plan.box_dst_slot[i]);
     for (size_t i = 0; i < plan.lists.size(); ++i)
+    {
+        // every level of every column once: the tiles of a group of levels take the columns in turn
+        const auto& l = plan.lists[i];
+        std::vector<char> seen((size_t)l.count * (size_t)l.levels, 0);
+        for (int k = plan.xb_list[i].first; k < plan.xb_list[i].first + plan.xb_list[i].second; ++k)
+        {
+            const xtile& t = plan.xb[k];
+            const int64_t level0 = l.s_ls ? (t.src - l.src) / ((int64_t)l.s_ls * l.unit) : 0;
+            for (uint32_t e = 0; e < t.count; ++e)
+            {
+                const auto [col, lev] = list_element(t, e);
+                if (col >= (uint32_t)l.count || level0 < 0 || level0 + lev >= (int64_t)l.levels || seen[(size_t)col * l.levels + (size_t)(level0 + lev)]++)
+                    throw error(GHEXB_ERR_INTERNAL, "a list's tiles differ from its columns");
+            }
+        }
+        if (std::find(seen.begin(), seen.end(), 0) != seen.end()) throw error(GHEXB_ERR_INTERNAL, "a list's tiles leave columns out");
         replay_range(plan.xb_list[i], plan.list_src_slot[i], plan.list_dst_slot[i]);
+    }
     // pairs: every element's source and destination, against the two boxes' own mapping
     for (size_t p = 0; p < plan.pairs.size(); ++p)
     {
@@ -1336,7 +1394,7 @@ int64_t check_tables(ghexb_plan_s& plan)
                 throw error(GHEXB_ERR_INTERNAL, "index block of a tile that has none");
             for (uint32_t e = 0; e < t.count; ++e)
             {
-                const uint32_t col = fast_div{t.n0, t.m0, t.l0}.div(t.e0 + e);
+                const uint32_t col = list_element(t, e).first;
                 const uint32_t c = col - (uint32_t)t.u0;
                 if (c >= (uint32_t)k_block_columns || blocks[p * k_block_ints + c] != t.sidx[col] ||
                     blocks[p * k_block_ints + k_block_columns + c] != t.didx[col])
@@ -1498,6 +1556,7 @@ int64_t check_tables(ghexb_plan_s& plan)
             if (t.kind == 1)
             {
                 covered += t.count;
+                check_list_elements(t);
                 if ((int64_t)t.col0 + (int64_t)(t.e0 + t.count - 1) / t.n0 * (t.nimg + 1) + t.nimg >= (int64_t)plan.lcols.size())
                     throw error(GHEXB_ERR_INTERNAL, "adjoint tile outside the column table");
             }

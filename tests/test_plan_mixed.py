@@ -1,7 +1,7 @@
 """Plans over patterns of different kinds (host replay, no GPU): fields of a regular grid whose short
 rows hold more lines than the L2, so that the batched tiles are placed field by field in bins, beside
-columns stored level by level, whose tiles start again for every group of levels. The fields are
-wrapped at fake addresses: nothing is dereferenced."""
+columns stored level by level, whose tiles start again for every group of levels, on their own and together.
+The fields are wrapped at fake addresses: nothing is dereferenced."""
 import ctypes as C
 import functools
 
@@ -37,6 +37,15 @@ def checked(ctx, handles):
     n = C.c_int64()
     _capi.call("ghexb_plan_check", ctx._h, (C.c_void_p * len(handles))(*handles), len(handles), C.byref(n))
     return n.value
+
+
+@pytest.mark.parametrize("levels", [1, 2, 30, 64, 65, 90, 300])
+def test_level_major_tiles(levels):
+    """Every halo level is checked in the forward, as an image of its owner and in the phased lists;
+    the replay takes the tiles' elements as the kernels do (columns of a group of levels in turn)."""
+    doms = W.config2(ni=40, nj=60, parts=4).domains
+    keep, handles = level_major_handles(doms, levels, 1 << 44)
+    assert checked(keep[0], handles) == 3 * levels * sum(outer.size for _, _, outer in doms)
 
 
 @functools.lru_cache(maxsize=1)
