@@ -2114,12 +2114,22 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
             const uint32_t col0 = group0 + (uint32_t)(nb * per);
             uint32_t gc = (uint32_t)(gather_per_thread(o0.nimg) * k_gather_block);
             const uint32_t n = (uint32_t)((int64_t)(b - a - nb) * o0.levels);
-            // levels further apart than columns (as the forward's list tiles): whole columns, as many
-            // as the block of column addresses holds, and neighbouring threads take neighbouring columns
-            // (16.1 -> 10.9 and 79.9 -> 56.8 us on the two sizes there)
-            const auto& of = plan.fields[o0.slot];
-            const bool by_column = o0.levels > 1 && of.level_stride > of.index_stride && (uint32_t)o0.levels <= gc;
-            if (by_column) gc = std::min(gc / (uint32_t)o0.levels, std::min<uint32_t>(32u, (uint32_t)k_gblock_entries / per)) * (uint32_t)o0.levels;
+            // Levels further apart than columns, in the owners' fields and the images' (as the forward's
+            // list tiles): whole columns, and neighbouring threads take neighbouring columns (16.1 ->
+            // 10.9 and 79.9 -> 56.8 us on the two sizes there). As many as the block of column addresses
+            // holds; where that gives more tiles than are resident at a time (4 per SM), as many as make
+            // one wave, but at most 1024 elements: few levels would leave most of a tile's threads idle.
+            // 64 domains of 2000 x 2000 columns, float64, by level / 32 columns / this: 4 levels 10.3 /
+            // 12.5 / 8.6 us, 8 levels 16.0 / 20.5 / 12.5, 12 levels 24.2 / 28.0 / 21.8, 30 levels 66.5 /
+            // 48.7 / 48.6; 16 of 512 x 768, 4 levels: 8.5 / 4.9 / 4.9 (in tiles of 1024 elements 6.2).
+            const auto apart = [&](int slot) { return plan.fields[slot].level_stride > plan.fields[slot].index_stride; };
+            const bool by_column = o0.levels > 1 && apart(o0.slot) && apart(o0.img_slot[0]) && (uint32_t)o0.levels <= gc;
+            if (by_column)
+            {
+                const uint32_t levels = (uint32_t)o0.levels, block = std::min<uint32_t>(32u, (uint32_t)k_gblock_entries / per);
+                const uint32_t wave = (uint32_t)((b - a - nb) / (4u * (uint32_t)(plan.ctx ? plan.ctx->num_sms : 148)));
+                gc = std::min(gc / levels, std::max(block, std::min(wave, 1024u / levels))) * levels;
+            }
             const fast_div f0 = fast_div::make((uint32_t)o0.levels);
             for (uint32_t e0 = 0; e0 < n; e0 += gc)
             {

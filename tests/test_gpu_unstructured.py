@@ -273,3 +273,17 @@ def test_level_major_tiles_bitexact(cuda, ni, nj, parts, levels):
             assert f[0].strides[1] > f[0].strides[0]
             (OU.adjoint if form == "adjoint" else OU.exchange)(recv, send, f)
             assert sum(bits_equal(a, e) for a, e in zip(g, f)) == 0
+
+
+@pytest.mark.parametrize("levels", [2, 5, 9])
+def test_level_major_adjoint_of_many_columns(cuda, levels):
+    """So many owner columns of few levels that a tile takes more of them than its block of column
+    addresses holds (64 domains of 1000 x 1000 columns: 54 owners of a tile)."""
+    w = W.config2(ni=1000, nj=1000, parts=64, levels=levels)
+    recv, send, _ = OU.make_pattern([OU.Domain(*d) for d in w.domains])
+    rng = np.random.default_rng(9)
+    fields = [[np.asfortranarray(rng.standard_normal((d[1].size, levels)).astype(t)) for d in w.domains] for t in (np.float64, np.float32)]
+    got = run_device(U.make_context(), w.domains, [[x.copy(order="K") for x in f] for f in fields], "adjoint")
+    for f, g in zip(fields, got):
+        OU.adjoint(recv, send, f)
+        assert sum(bits_equal(a, e) for a, e in zip(g, f)) == 0
