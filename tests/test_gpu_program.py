@@ -17,6 +17,7 @@ from ghex_b200 import _capi
 from ghex_b200 import autograd as AG
 from ghex_b200 import workloads as W
 from ghex_b200._capi import GhexError
+from ghex_b200.structured import regular as R
 
 from gpu_helpers import RegularRun, bits_equal
 
@@ -90,6 +91,36 @@ def test_fused_program_bits(cuda, shape, parts, periodic, halo, seed, dtype):
         assert equal(*ins)
         assert equal(*grads)
     assert dx._program(halo).status() == 0
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_fused_program_of_other_orders(cuda, seed):
+    """Two fields on uneven domains, of one pattern or two, given in any order, each in a memory order
+    of its own: the images of a cell are added in the order of the exchange's adjoint."""
+    rng = np.random.default_rng(seed)
+    shape, parts, periodic = (31, 24, 20), (3, 2, 2), tuple(bool(v) for v in rng.integers(0, 2, 3))
+    dtype = (torch.float64, torch.float32)[seed % 2]
+    doms = W.regular_decomposition(shape, parts, seed)
+    ctx = R.make_context()
+    descs = [R.DomainDescriptor(i, (f, l)) for i, f, l in doms]
+    hg = R.HaloGenerator(((0, 0, 0), tuple(n - 1 for n in shape)), (1, 1, 1), periodic)
+    patterns = [R.make_pattern(ctx, hg, descs) for _ in range(2 if seed % 3 else 1)]
+    gen = torch.Generator(device=cuda).manual_seed(seed)
+    bound = []
+    for which in range(2):
+        for d, dd in zip(doms, descs):
+            ext = tuple(d[2][k] - d[1][k] + 3 for k in range(3))
+            order = rng.permutation(3)
+            x = torch.empty([ext[k] for k in order], dtype=dtype, device=cuda).uniform_(-1, 1, generator=gen)
+            x = x.permute([int(k) for k in np.argsort(order)])
+            bound.append((patterns[which % len(patterns)](R.make_field_descriptor(dd, x, (1, 1, 1), ext)), x))
+    if seed:
+        # (fields of one pattern are paired over the domains in the order given: the first field's before the second's)
+        keep = rng.permutation(len(doms))
+        bound = [bound[i] for i in keep] + [bound[len(doms) + i] for i in rng.permutation(len(doms))]
+    dx = AG.DifferentiableExchange(ctx, [b for b, _ in bound])
+    assert dx._program(1) is not None
+    check_fields_and_gradients(cuda, dx, [x for _, x in bound], 3, 1, 1)
 
 
 def check_fields_and_gradients(cuda, dx, x0, steps, halo, repeats):
