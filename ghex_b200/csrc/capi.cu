@@ -1122,8 +1122,29 @@ int ghexb_program_steps(ghexb_program program, const void* const* fields, const 
         {
             require(!fields || (fields[i] && aligned(fields[i], es)), "a field is null or not aligned to its element size");
             require(!out || (out[i] && aligned(out[i], es)), "an output is null or not aligned to its element size");
-            // the output of a single pass must not be its input
-            require(!fields || !out || steps > 1 || fields[i] != out[i], "input and output overlap");
+        }
+        // a single pass reads its fields, and their neighbours, while it writes its outputs
+        if (fields && out && steps == 1)
+        {
+            std::vector<std::array<uintptr_t, 3>> spans; // first byte, end, output or not
+            for (size_t i = 0; i < n; ++i)
+            {
+                const auto& d = program->domains[i];
+                int64_t bytes = (int64_t)es;
+                for (int k = 0; k < 3; ++k) bytes += (d.n[k] + 2 * program->halo - 1) * d.s[k] * (int64_t)es;
+                for (const uintptr_t kind : {uintptr_t(0), uintptr_t(1)})
+                {
+                    const auto p = reinterpret_cast<uintptr_t>(kind ? out[i] : fields[i]);
+                    spans.push_back({p, p + (uintptr_t)bytes, kind});
+                }
+            }
+            std::sort(spans.begin(), spans.end());
+            uintptr_t end[2] = {0, 0}; // of the fields and of the outputs so far
+            for (const auto& s : spans)
+            {
+                require(s[0] >= end[1 - s[2]], "input and output overlap");
+                end[s[2]] = std::max(end[s[2]], s[1]);
+            }
         }
         const int packed = steps - (out ? 1 : 0); // passes that write a packed buffer
         require(packed < 1 || ((source == a ? b : a) != nullptr), "a packed buffer is missing");

@@ -357,3 +357,18 @@ def test_a_pass_that_gave_up_is_reported(cuda):
     assert equal(AG.diffusion_program(dx, [x.clone() for x in x0], 2, ALPHA), ys)
     word[0] = 1
     assert dx._program(1).status() == 1 and dx._program(1).status() == 0
+
+
+def test_a_single_pass_out_of_place(cuda):
+    """One step reads a domain's neighbours while it writes: no output may lie in any field."""
+    dx, x0 = make(cuda, (12, 10, 8), (2, 1, 1), (True, True, True), 1, np.float64, None)
+    program, stream = dx._program(1), torch.cuda.current_stream()
+    before = [x.clone() for x in x0]
+    fresh = torch.empty_like(x0[0])
+    for out in (x0, [fresh, x0[0]], [x0[1], fresh]):
+        with pytest.raises(GhexError, match="overlap"):
+            program.steps(1, ALPHA, stream, fields=x0, out=out)
+    assert equal(x0, before)
+    out = [torch.empty_like(x) for x in x0]
+    program.steps(1, ALPHA, stream, fields=x0, out=out)
+    assert equal(out, separately(dx, before, 1, 1)[1])
