@@ -783,7 +783,8 @@ def measure_program(dev, timer, dtype, steps, warmup, baseline=True) -> dict:
            "forward_backward_ms": ms_fb, "forward_ms": ms_f, "inner_steps": nsteps,
            "forward_backward_ms_per_inner_step": ms_fb / nsteps, "plan_pool": dx.pool_stats(),
            "graphed": {"forward_backward_ms": ms_graph, "forward_backward_ms_per_inner_step": ms_graph / nsteps,
-                       "form": "GraphedDiffusion: the same kernels in one CUDA graph on fixed buffers",
+                       "form": "GraphedDiffusion: the first fused pass launched on the inputs, the others, the loss and the "
+                               "backward's passes replayed from one CUDA graph on fixed buffers",
                        "same_bits_as_autograd": bool(bits(loss_g, loss_a) and all(bits(g, a) for g, a in zip(grad_g, out["grad"])))}}
     if baseline:
         from oracle import regular as O

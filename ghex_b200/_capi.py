@@ -168,7 +168,6 @@ for _name, _args in SIGNATURES.items():
 # The calls of an exchange, bound once; the field handles are given by the address of an array of them.
 co_exchange = C.CFUNCTYPE(C.c_int, _vp, _vp, _i, _vp, C.POINTER(_vp))(("ghexb_co_exchange", lib))
 handle_wait = lib.ghexb_handle_wait
-handle_destroy = lib.ghexb_handle_destroy
 
 
 class GhexError(RuntimeError):

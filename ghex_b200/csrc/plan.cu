@@ -1988,8 +1988,14 @@ void build_tiles(ghexb_plan_s& plan, const int32_t* idx)
             // whose short rows alone hold more lines than the L2 goes in bins of the same fraction of
             // every descriptor (the same rows and levels of every face): cubed sphere of edge 384, 90
             // levels, 178 -> 163 us (DRAM reads 369 -> 323 MB, the distinct lines 313 MB); four bins where
-            // a field's lines fit cost the regular case 174 us. (400 x 300 x 96, whose lines of 79 MB fit,
-            // takes 62 us either way.)
+            // a field's lines fit cost the regular case 174 us.
+            // The line at 96 MB, by cost / by field: five fields of 400 x 300 x 96 (80 MB) 61.7 / 60.6 us,
+            // 300 x 200 x 64 (37 MB) 36.5 / 38.1, 600 x 450 x 144 (175 MB) 117 / 107, 300 x 480 x 160 (311
+            // MB) 162 / 138; cubed sphere, float64, edge 192 (292 MB) 95.9 / 88.7, 256 (385 MB) 122.6 /
+            // 112.3, 320 (478 MB) 149.4 / 136.2. It loses on five float64 fields in 2 x 2 x 2 domains of 640 x
+            // 480 x 160 (102 MB: 100.8 / 102.3) and on a scalar and a vector in float32 on cubes of edge
+            // 320 and more (121.0 / 123.0, edge 384 140.9 / 146.7; in bins of 48 MB 119.2 and 142.7, which
+            // cost the regular cases 1 %).
             std::vector<uint32_t> bins(lines.size()), first(lines.size() + 1, 0); // bins of a field, the first of them
             for (size_t f = 0; f < lines.size(); ++f) bins[f] = 1 + (uint32_t)(lines[f] / k_order_bytes), first[f + 1] = first[f] + bins[f];
             std::vector<uint32_t> at(first.back() + 1, 0), bin(all.size());

@@ -7,6 +7,9 @@
 // exchange's adjoint would have added from each of its images, in the same order. Every value is
 // the one that the exchange kernel and the stencil kernel (stencil.cu) compute one after the
 // other, with the same roundings, so results have the same bits.
+// (One exception: images of halo cells that no interior cell lies beside are zeros, which a pass
+// leaves out and the exchange's adjoint adds. Where that is all that is added to a cell, a zero may
+// keep the minus sign that a negative alpha gave it.)
 //
 // The fields between two passes are the program's own, and packed: interiors only, rows on
 // 32-byte boundaries, so that a thread moves 16 bytes at a time whatever the domains' extents.
@@ -133,6 +136,7 @@ template <typename T> __device__ __forceinline__ void not_a_number(cells<T>& a)
 __device__ __forceinline__ void report(unsigned* status) { *reinterpret_cast<volatile unsigned*>(status) = 1u; }
 
 constexpr int k_batch = 32; // domains per launch
+constexpr int k_sms = 148;  // of a B200
 
 // Passes follow one another: a pass lets the next one be launched (programmatic stream serialisation)
 // when its blocks come to their last plane, so that the other's blocks start and set up their
@@ -786,7 +790,7 @@ int slabs_of(uint64_t groups, int nz, int per_sm)
     double least = 0;
     for (int s = 1; s <= std::max(1, nz / k_min_slab); ++s)
     {
-        const double blocks = (double)(groups * s), resident = 148.0 * per_sm;
+        const double blocks = (double)(groups * s), resident = (double)k_sms * per_sm;
         const double waves = blocks <= resident ? 1.0 : (double)(int64_t)((blocks + resident - 1) / resident);
         const double planes = waves * ((nz + s - 1) / s + 3);
         if (s == 1 || planes < least) best = s, least = planes;

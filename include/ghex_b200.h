@@ -405,8 +405,9 @@ int ghexb_program_buffer_bytes(ghexb_program program, int64_t* bytes);
  * the exchange and the update, with the output halo 0. adjoint != 0: a pass is the update's
  * transpose and the exchange's adjoint. twice != 0 (adjoint, from `source`): the source times two,
  * the gradient of its sum of squares. alpha must be finite in the fields' type (with another one
- * the gradients of halo edges, which the passes leave out, are not zero). Results have the bits of ghexb_plan_launch and
- * ghexb_stencil7 (or of the latter's transpose and ghexb_plan_adjoint_launch) in turn. */
+ * the gradients of halo edges, which the passes leave out, are not zero). Results have the bits of
+ * ghexb_plan_launch and ghexb_stencil7 (or of the latter's transpose and ghexb_plan_adjoint_launch)
+ * in turn, but for the sign of zeros in the transpose with a negative alpha. */
 int ghexb_program_steps(ghexb_program program, const void* const* fields, const void* source, void* const* out, void* a,
                         void* b, int steps, double alpha, int adjoint, int twice, void* stream);
 /* Sum of squares of the interiors of n 3-D arrays (arguments as ghexb_stencil7's), added in 64
